@@ -473,7 +473,7 @@ int lsg_row_classes(lsg_ctx* ctx, int level, int* cls, double* dict, int* nclass
 /* Solve A x = b; x holds the initial guess on entry and the solution on exit
    (IterativeSolverInterface::solve).  Host buffers of N*M*K doubles.
    The first preconditioner application after lsg_setup records the
-   multigrid V-cycle (or the ILU(0) sweeps) as a CUDA graph on the
+   multigrid V-cycle as a CUDA graph on the
    context's own stream and later ones replay it; make that first solve
    outside any stream capture of the caller's. */
 int lsg_solve(lsg_ctx* ctx, const double* b, double* x, lsg_stats* stats);
@@ -566,13 +566,13 @@ int lsg_mg_level_tridiag(lsg_ctx* ctx, int level, char dir, double* c, double* d
    lsg_setup with the multigrid preconditioner. */
 int lsg_profile_kernel(lsg_ctx* ctx, int which, int reps, double* ms_per_launch, double* bytes_per_launch);
 
-/* Self-test of the bounded waits: runs the one-launch ILU(0) sweep of an
-   ILU(0) context with one CTA leaving before its first barrier arrival, so
-   the other CTAs' first wait runs out (after about one second) and the
-   kernel returns with its error flag set.  Returns LSG_ERR_CUDA with
+/* Self-test of the bounded waits: runs an ILU(0) application of an ILU(0)
+   context in which the first tile's CTA leaves without writing its face
+   values, so the waits of the CTAs next to it run out (after about one
+   second) and the kernel returns with its error flag set.  Returns LSG_ERR_CUDA with
    lsg_last_error describing it (the expected result); the context stays
    usable.  Needs lsg_setup with LSG_PC_ILU0 on a grid whose sweep has two
-   CTAs or more. */
+   tiles of 16 x 16 lines in (y, z) or more. */
 int lsg_selftest_wait_limit(lsg_ctx* ctx);
 
 /* Residual r = b - A x and its squared 2-norm for a 7-point operator given

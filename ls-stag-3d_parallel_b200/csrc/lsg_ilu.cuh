@@ -8,10 +8,9 @@
 //     U_kj = A_kj                   j in {e, n, t}
 // so only the pivots U_kk need computing; they depend on the three upstream
 // neighbours, i.e. on the previous hyperplane x + y + z = const.  The
-// triangular solves sweep the same hyperplanes
-// (ILUDecomposition7pStencilMatrix::DirectGauss/InverseGauss,
-// ilu_decomposition_7p_stencil_matrix.h:90-134), one launch per hyperplane,
-// all captured in one CUDA graph.
+// triangular solves (ILUDecomposition7pStencilMatrix::DirectGauss/InverseGauss,
+// ilu_decomposition_7p_stencil_matrix.h:90-134) have the same dependencies;
+// they run as a pipeline of tiles of x-lines (k_ilu_tile_sweep).
 #pragma once
 
 #include "lsg_kernels.cuh"
@@ -29,6 +28,12 @@ __device__ __forceinline__ bool plane_cell(int level, long long t, int N, int M,
     if (z < 0 || z >= K) return false;
     i = (long long)z * N * M + (long long)y * N + x;
     return true;
+}
+
+// the divisor U_jj of a lower coefficient, kept away from 0
+__device__ __forceinline__ double ilu_clamp(double u)
+{
+    return fabs(u) < 1e-12 ? ((u < 0.0) ? -1e-12 : 1e-12) : u;
 }
 
 // Pivots of one hyperplane.  A: 7 planes b s w p e n t; U: pivot array.
@@ -134,177 +139,379 @@ __global__ void k_ilu_bwd(int level, int N, int M, int K, const double* __restri
     }
 }
 
-// Grid-wide barrier of the cooperative ILU sweep (every CTA resident):
-// arrivals are counted on bar[0] (zeroed before the launch); it gives up
-// after one second, setting *err.  Values other CTAs wrote before the
-// barrier are read after it through L2 (__ldcg).
-__device__ __forceinline__ bool ilu_grid_barrier(unsigned int* bar, unsigned int target, int* err)
+// ---------------------------------------------------------------------------
+// The triangular solves as a pipeline of tiles.
+//
+// The grid's x-lines are cut into tiles of 16 x 16 lines in (y, z), one CTA
+// per tile, one thread per line.  At step s the thread of line (ty, tz) works
+// on cell x = s - ty - tz, so the cells of one step lie on one hyperplane, the
+// values of a line's lower neighbours were computed one step earlier by this
+// thread (x - 1) and by the threads next to it (y - 1, z - 1, through shared
+// memory), and a step costs one barrier of one CTA.  Only the tile's two
+// faces are exchanged between CTAs.
+//
+// Storage follows the steps: position (tile, step, thread), so that every
+// stream is contiguous in the order in which it is used.  A tile has
+// S = N + 30 steps, rounded up to whole chunks of kIluC; positions outside
+// the grid hold zeros.
+// ---------------------------------------------------------------------------
+constexpr int kIluTY = 16, kIluTZ = 16, kIluT = kIluTY * kIluTZ;
+constexpr int kIluC = 4;                  // steps per chunk
+constexpr int kIluSlots = 3;              // chunks of factors and right-hand side in flight
+constexpr int kIluFaceSlots = 4;          // chunks of face values in flight
+constexpr int kIluThreads = kIluT + 64;   // line threads, the loading warp, the face warp
+
+struct IluTiles {
+    int N, M, K;
+    int nty, ntz;                         // tiles in y and z
+    int nc;                               // chunks per tile
+    long long steps() const { return (long long)nc * kIluC; }
+    long long positions() const { return (long long)nty * ntz * steps() * kIluT; }
+};
+
+inline IluTiles ilu_tiles(int N, int M, int K)
 {
+    IluTiles g;
+    g.N = N;
+    g.M = M;
+    g.K = K;
+    g.nty = (M + kIluTY - 1) / kIluTY;
+    g.ntz = (K + kIluTZ - 1) / kIluTZ;
+    g.nc = (N + kIluTY + kIluTZ - 2 + kIluC - 1) / kIluC;
+    return g;
+}
+
+// Coefficients per position: L_b, L_s, L_w of the forward sweep; U_e, U_n,
+// U_t, U_p and 1 / U_p of the backward sweep, stored as [tile][chunk][kind]
+// [step of the chunk][thread].
+constexpr int kIluFwd = 3, kIluBwd = 5;
+
+// Fills both coefficient arrays from the operator's planes and the pivots
+// (L_kj = A_kj / clamp(U_jj), U_kj = A_kj); one thread per position.
+__global__ void k_ilu_tile_factors(IluTiles g, const double* __restrict__ A, const double* __restrict__ U,
+                                   double* __restrict__ facL, double* __restrict__ facU)
+{
+    const long long n = (long long)g.N * g.M * g.K;
+    const long long NM = (long long)g.N * g.M;
+    const long long S = (long long)g.nc * kIluC, total = (long long)g.nty * g.ntz * S * kIluT;
+    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < total;
+         q += (long long)gridDim.x * blockDim.x) {
+        const int t = (int)(q % kIluT);
+        const long long ts = q / kIluT;                   // tile * S + step
+        const int step = (int)(ts % S), tile = (int)(ts / S);
+        const int ty = t % kIluTY, tz = t / kIluTY;
+        const int x = step - ty - tz, y = (tile % g.nty) * kIluTY + ty, z = (tile / g.nty) * kIluTZ + tz;
+        double l[kIluFwd] = {0, 0, 0}, u[kIluBwd] = {0, 0, 0, 0, 0};
+        if (x >= 0 && x < g.N && y < g.M && z < g.K) {
+            const long long i = x + g.N * ((long long)y + (long long)g.M * z);
+            if (z > 0) l[0] = A[i] / ilu_clamp(U[i - NM]);
+            if (y > 0) l[1] = A[n + i] / ilu_clamp(U[i - g.N]);
+            if (x > 0) l[2] = A[2 * n + i] / ilu_clamp(U[i - 1]);
+            if (x < g.N - 1) u[0] = A[4 * n + i];
+            if (y < g.M - 1) u[1] = A[5 * n + i];
+            if (z < g.K - 1) u[2] = A[6 * n + i];
+            u[3] = U[i];
+            u[4] = 1.0 / U[i];
+        }
+        const long long chunk = (long long)tile * g.nc + step / kIluC;
+        const int in = (step % kIluC) * kIluT + t;
+        for (int k = 0; k < kIluFwd; k++) facL[(chunk * kIluFwd + k) * kIluC * kIluT + in] = l[k];
+        for (int k = 0; k < kIluBwd; k++) facU[(chunk * kIluBwd + k) * kIluC * kIluT + in] = u[k];
+    }
+}
+
+// A vector of the grid into the tiles' step order (IN) or back: a CTA takes 32
+// steps of 64 of a tile's lines through shared memory, so that both sides move
+// whole 256-byte rows.  Positions outside the grid are set to 0.
+template <bool IN>
+__global__ void __launch_bounds__(256) k_ilu_tile_vector(IluTiles g, const double* __restrict__ src,
+                                                          double* __restrict__ dst)
+{
+    __shared__ double sm[64][33];
+    const int S = g.nc * kIluC;
+    const int s0 = blockIdx.y * 32, zg = blockIdx.z, tile = blockIdx.x;
+    const int y0 = (tile % g.nty) * kIluTY, z0 = (tile / g.nty) * kIluTZ + zg * 4;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int l0 = threadIdx.x & 63, u0 = threadIdx.x >> 6;
+    const long long base = ((long long)tile * S + s0) * kIluT + zg * 64;
+    auto rows = [&](auto&& body) {                        // the CTA's lines along x: one warp a line
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int l = wid + 8 * k, ty = l & 15, tz = zg * 4 + (l >> 4);
+            const int x = s0 + lane - ty - tz, y = y0 + ty, z = z0 + (l >> 4);
+            const bool in = x >= 0 && x < g.N && y < g.M && z < g.K;
+            body(l, in, x + g.N * ((long long)y + (long long)g.M * z));
+        }
+    };
+    if (IN) {
+        rows([&](int l, bool in, long long i) { sm[l][lane] = in ? src[i] : 0.0; });
+        __syncthreads();
+#pragma unroll
+        for (int u = u0; u < 32; u += 4)
+            if (s0 + u < S) dst[base + (long long)u * kIluT + l0] = sm[l0][u];
+    } else {
+#pragma unroll
+        for (int u = u0; u < 32; u += 4)
+            sm[l0][u] = s0 + u < S ? src[base + (long long)u * kIluT + l0] : 0.0;
+        __syncthreads();
+        rows([&](int l, bool in, long long i) {
+            if (in) dst[i] = sm[l][lane];
+        });
+    }
+}
+
+__device__ __forceinline__ unsigned long long ilu_now()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ unsigned ilu_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void ilu_mbar_arrive(unsigned long long* bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(ilu_smem(bar)) : "memory");
+}
+
+// Waits for the phase of `bar` with this parity, for four seconds at most (the
+// face warp's polls, which these waits depend on, end after one): then the
+// error flag is set and the kernel runs on without waiting (wrong values,
+// reported by the solve), so no thread is left behind at a barrier.
+__device__ __forceinline__ void ilu_mbar_wait(unsigned long long* bar, unsigned parity, int* err, bool& gave_up)
+{
+    unsigned long long t0 = 0;
+    for (unsigned it = 0; !gave_up; it++) {
+        unsigned ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(ilu_smem(bar)), "r"(parity)
+            : "memory");
+        if (ok) break;
+        if ((it & 63) == 0) {
+            const unsigned long long now = ilu_now();
+            if (it == 0) t0 = now;
+            else if (now - t0 > 4000000000ull) {
+                atomicExch(err, 1);
+                gave_up = true;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void ilu_bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     ilu_smem(dst)),
+                 "l"(src), "r"(bytes), "r"(ilu_smem(bar))
+                 : "memory");
+}
+
+// A face value in global memory: the two halves of the double, each beside the
+// sweep's tag, so the reader knows from the words themselves that the value is
+// there (8-byte words are written whole) and neither side needs a fence.
+__device__ __forceinline__ void ilu_face_store(uint4* p, double v, unsigned tag)
+{
+    const unsigned lo = (unsigned)__double2loint(v), hi = (unsigned)__double2hiint(v);
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p),
+                 "l"(((unsigned long long)tag << 32) | lo), "l"(((unsigned long long)tag << 32) | hi)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool ilu_face_load(const uint4* p, double& v, unsigned tag)
+{
+    unsigned long long a, b;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+    v = __hiloint2double((int)(unsigned)b, (int)(unsigned)a);
+    return (unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag;
+}
+
+template <bool FWD>
+constexpr size_t ilu_sweep_smem()
+{
+    return sizeof(double) * ((size_t)kIluSlots * ((FWD ? kIluFwd : kIluBwd) + 1) * kIluC * kIluT +
+                             (size_t)kIluFaceSlots * kIluC * 32 + 2 * kIluT) +
+           8 * (2 * kIluSlots + 2 * kIluFaceSlots);
+}
+
+// One triangular sweep, in place on the tile-ordered vector v: forward
+// y = b - (L_b y_b + L_s y_s + L_w y_w), or backward
+// x = (y - (U_e x_e + U_n x_n + U_t x_t)) / U_p, the terms in that order.
+//
+// A CTA takes its tile from a ticket, in the order of the tiles' diagonals, so
+// every tile it depends on is held by a CTA that started before it and no CTA
+// waits for one that has not.  The loading warp brings chunks of coefficients
+// and right-hand sides (contiguous) into a ring in shared memory with bulk
+// copies; the face warp polls the two upstream tiles' face values of a chunk
+// and puts them into a ring of their own, one lane per face line; the line
+// threads take kIluC steps per chunk.  Every wait ends after a second
+// (ilu_mbar_wait); withhold >= 0 (the wait-limit self-test only): the CTA
+// with that ticket leaves at once and writes no face.
+//
+// The quotient by U_p comes from the rounded reciprocal r = 1 / U_p and one
+// remainder step, q0 = a r, q = q0 + (a - q0 U_p) r, which rounds as the
+// division does (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), in three
+// dependent operations instead of a division in the recurrence.
+template <bool FWD>
+__global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, const int* __restrict__ order,
+                                                                 const double* __restrict__ fac, double* v,
+                                                                 uint4* faces, unsigned tag, unsigned* ticket,
+                                                                 unsigned base, int* err, int withhold)
+{
+    constexpr int NK = FWD ? kIluFwd : kIluBwd;
+    constexpr int CT = kIluC * kIluT;
+    extern __shared__ __align__(128) unsigned char ilu_sm_raw[];
+    double* ilu_sm = reinterpret_cast<double*>(ilu_sm_raw);
+    double* ring = ilu_sm;                                        // [slot][kind, then v][step][thread]
+    double* fring = ring + (size_t)kIluSlots * (NK + 1) * CT;     // [slot][step][32 face lines]
+    double* sh = fring + kIluFaceSlots * kIluC * 32;              // [2][thread]
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(sh + 2 * kIluT);
+    unsigned long long* empty = full + kIluSlots;
+    unsigned long long* ffull = empty + kIluSlots;
+    unsigned long long* fempty = ffull + kIluFaceSlots;
+    __shared__ unsigned my;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        my = atomicAdd(ticket, 1u) - base;                        // base: the tickets of the earlier launches
+        for (int k = 0; k < kIluSlots; k++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(full + k)), "r"(1) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(empty + k)), "r"(kIluT / 32)
+                         : "memory");
+        }
+        for (int k = 0; k < kIluFaceSlots; k++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(ffull + k)), "r"(1) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(fempty + k)), "r"(kIluT / 32)
+                         : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid < kIluT) sh[tid] = sh[kIluT + tid] = 0.0;
     __syncthreads();
-    __shared__ int ok;
-    if (threadIdx.x == 0) {
-        // arrive (release: this CTA's stores first), then poll with acquire
-        // loads; every 256 polls look at the clock and at the error flag
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-        ok = 1;
-        unsigned long long t0 = 0;
-        for (unsigned it = 0;; it++) {
-            unsigned int v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (v >= target) break;
-            if ((it & 255) == 0) {
-                unsigned long long now;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-                if (it == 0) t0 = now;
-                else if (now - t0 > 1000000000ull || *(volatile int*)err != 0) {
-                    atomicExch(err, 1);
-                    ok = 0;
-                    break;
+    if ((int)my == withhold) return;
+    const int ntile = g.nty * g.ntz;
+    const int tile = order[FWD ? (int)my : ntile - 1 - (int)my];
+    const int ta = tile % g.nty, tb = tile / g.nty;
+    const int nc = g.nc, S = nc * kIluC;
+    bool gave_up = false;
+
+    if (warp == kIluT / 32) {                                     // the loading warp
+        if (lane != 0) return;
+        for (int c = 0; c < nc; c++) {
+            const int slot = c % kIluSlots, cf = FWD ? c : nc - 1 - c;
+            if (c >= kIluSlots) {
+                ilu_mbar_wait(empty + slot, (unsigned)(c / kIluSlots - 1) & 1u, err, gave_up);
+                bool late = false;                                // a slot's copies end before the next ones start
+                if (gave_up) ilu_mbar_wait(full + slot, (unsigned)(c / kIluSlots - 1) & 1u, err, late);
+            }
+            double* dst = ring + (size_t)slot * (NK + 1) * CT;
+            const long long chunk = (long long)tile * nc + cf;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ilu_smem(full + slot)),
+                         "r"((unsigned)((NK + 1) * CT * sizeof(double)))
+                         : "memory");
+            ilu_bulk_load(dst, fac + chunk * NK * CT, NK * CT * sizeof(double), full + slot);
+            ilu_bulk_load(dst + NK * CT, v + chunk * CT, CT * sizeof(double), full + slot);
+        }
+        for (int c = max(0, nc - kIluSlots); c < nc; c++) {       // no copy outlives the CTA
+            bool late = false;
+            ilu_mbar_wait(full + c % kIluSlots, (unsigned)(c / kIluSlots) & 1u, err, late);
+        }
+        return;
+    }
+    if (warp == kIluT / 32 + 1) {                                 // the face warp
+        // lanes 0..15: the y-face line tz = lane of the tile before (FWD) or
+        // after in y; lanes 16..31: the z-face line ty = lane - 16
+        const bool yf = lane < 16;
+        const bool has = FWD ? (yf ? ta > 0 : tb > 0) : (yf ? ta + 1 < g.nty : tb + 1 < g.ntz);
+        const int up = tile + (FWD ? -1 : 1) * (yf ? 1 : g.nty);
+        const uint4* src = faces + (long long)(has ? up : tile) * S * 32 + lane;
+        for (int c = 0; c < nc; c++) {
+            const int slot = c % kIluFaceSlots, s0 = (FWD ? c : nc - 1 - c) * kIluC;
+            if (c >= kIluFaceSlots)
+                ilu_mbar_wait(fempty + slot, (unsigned)(c / kIluFaceSlots - 1) & 1u, err, gave_up);
+            gave_up = __any_sync(0xffffffffu, gave_up);
+            double val[kIluC];
+            unsigned long long t0 = 0;
+            for (unsigned it = 0;; it++) {
+                bool ok = true;
+#pragma unroll
+                for (int u = 0; u < kIluC; u++) {
+                    const int st = s0 + u + (FWD ? 15 : -15);     // the upstream tile's step of the same cell column
+                    val[u] = 0.0;
+                    if (has && st >= 0 && st < S) ok = ilu_face_load(src + (long long)st * 32, val[u], tag) && ok;
+                }
+                if (__all_sync(0xffffffffu, ok) || gave_up) break;
+                if ((it & 63) == 0) {
+                    const unsigned long long now = ilu_now();
+                    if (it == 0) t0 = now;
+                    else if (now - t0 > 1000000000ull || *(volatile int*)err != 0) gave_up = true;
+                    gave_up = __any_sync(0xffffffffu, gave_up);
+                    if (gave_up && lane == 0) atomicExch(err, 1);
                 }
             }
-        }
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
-// Position of cell (x, y, z) in the hyperplane order: planes l = x + y + z in
-// turn, inside a plane by z, then y (x = l - y - z).  start[l] is the first
-// position of plane l, rowstart[l K + z] the first of its row z.
-__device__ __forceinline__ int ilu_hpos(int x, int y, int z, int N, int K, const int* __restrict__ start,
-                                        const int* __restrict__ rowstart)
-{
-    const int l = x + y + z;
-    const int ymin = max(0, l - z - (N - 1));
-    return start[l] + rowstart[(long long)l * K + z] + (y - ymin);
-}
-
-// The factors and neighbour positions in hyperplane order: perm[p] = i for
-// the cell i at position p; fac = L_b, L_s, L_w, U_e, U_n, U_t, U_p (7 arrays
-// of n); nbr = the positions of the cells below (z-1, y-1, x-1) and above
-// (x+1, y+1, z+1), -1 outside the grid (6 arrays of n).
-__global__ void k_ilu_perm_build(int N, int M, int K, const int* __restrict__ start, const int* __restrict__ rowstart,
-                                 const double* __restrict__ Lp, const double* __restrict__ A,
-                                 const double* __restrict__ U, int* __restrict__ perm, double* __restrict__ fac,
-                                 int* __restrict__ nbr)
-{
-    const long long n = (long long)N * M * K;
-    const int NM = N * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        cell_xyz(i, N, NM, x, y, z);
-        const int p = ilu_hpos(x, y, z, N, K, start, rowstart);
-        perm[p] = (int)i;
-        fac[p] = Lp[i];
-        fac[n + p] = Lp[n + i];
-        fac[2 * n + p] = Lp[2 * n + i];
-        fac[3 * n + p] = A[4 * n + i];
-        fac[4 * n + p] = A[5 * n + i];
-        fac[5 * n + p] = A[6 * n + i];
-        fac[6 * n + p] = U[i];
-        nbr[p] = z > 0 ? ilu_hpos(x, y, z - 1, N, K, start, rowstart) : -1;
-        nbr[n + p] = y > 0 ? ilu_hpos(x, y - 1, z, N, K, start, rowstart) : -1;
-        nbr[2 * n + p] = x > 0 ? ilu_hpos(x - 1, y, z, N, K, start, rowstart) : -1;
-        nbr[3 * n + p] = x < N - 1 ? ilu_hpos(x + 1, y, z, N, K, start, rowstart) : -1;
-        nbr[4 * n + p] = y < M - 1 ? ilu_hpos(x, y + 1, z, N, K, start, rowstart) : -1;
-        nbr[5 * n + p] = z < K - 1 ? ilu_hpos(x, y, z + 1, N, K, start, rowstart) : -1;
-    }
-}
-
-// Both triangular sweeps of one ILU(0) application in one cooperative launch
-// over the hyperplane-ordered factors (k_ilu_perm_build): the cells of a
-// plane are contiguous, so every stream of a plane is read coalesced, and
-// their neighbours in the previous plane lie close together.  Each thread
-// takes positions t, t + T, ... (at most CMAX) of every plane, with the
-// arithmetic of k_ilu_fwd / k_ilu_bwd (the same bits); b is gathered and x
-// scattered through perm inside the sweeps.  A plane's operands that do not
-// depend on the previous plane are loaded before the barrier that ends it.
-template <int CMAX>
-__global__ void __launch_bounds__(256) k_ilu_sweep_perm(int planes, long long n, const int* __restrict__ start,
-                                                         const int* __restrict__ perm, const double* __restrict__ fac,
-                                                         const int* __restrict__ nbr, const double* __restrict__ b,
-                                                         double* yp, double* xp, double* __restrict__ x,
-                                                         unsigned int* bar, int* err, int withhold)
-{
-    // withhold >= 0 (the wait-limit self-test only): that CTA leaves before its
-    // first barrier arrival, so the others' first wait runs out
-    if ((int)blockIdx.x == withhold) return;
-    const int T = gridDim.x * blockDim.x;                 // T * CMAX >= the largest plane (host)
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    int pos[CMAX], n0[CMAX], n1[CMAX], n2[CMAX];
-    double v0[CMAX], v1[CMAX], v2[CMAX], v3[CMAX], v4[CMAX];
-    auto fwd_operands = [&](int level) {
-        const int s0 = start[level], cnt = start[level + 1] - s0;
 #pragma unroll
-        for (int k = 0; k < CMAX; k++) {
-            const int q = tid + k * T;
-            pos[k] = q < cnt ? s0 + q : -1;
-            if (pos[k] >= 0) {
-                const int p = pos[k];
-                v0[k] = b[perm[p]];
-                v1[k] = fac[p];
-                v2[k] = fac[n + p];
-                v3[k] = fac[2 * n + p];
-                n0[k] = nbr[p];
-                n1[k] = nbr[n + p];
-                n2[k] = nbr[2 * n + p];
+            for (int u = 0; u < kIluC; u++) fring[(slot * kIluC + u) * 32 + lane] = val[u];
+            __syncwarp();
+            if (lane == 0) ilu_mbar_arrive(ffull + slot);
+        }
+        return;
+    }
+
+    // the line threads
+    const int ty = tid % kIluTY, tz = tid / kIluTY;
+    const bool edge_y = FWD ? ty == 0 : ty == kIluTY - 1, edge_z = FWD ? tz == 0 : tz == kIluTZ - 1;
+    // this line is a face that the downstream tiles read
+    const bool out_y = FWD ? ty == kIluTY - 1 : ty == 0, out_z = FWD ? tz == kIluTZ - 1 : tz == 0;
+    uint4* face = faces + (long long)tile * S * 32;
+    double* vt = v + (long long)tile * S * kIluT + tid;
+    double own = 0.0;                                             // the line's previous value
+    int p = 0;
+    for (int c = 0; c < nc; c++) {
+        const int slot = c % kIluSlots, fslot = c % kIluFaceSlots;
+        const int s0 = (FWD ? c : nc - 1 - c) * kIluC;
+        ilu_mbar_wait(full + slot, (unsigned)(c / kIluSlots) & 1u, err, gave_up);
+        const double* in = ring + (size_t)slot * (NK + 1) * CT + tid;
+        double a[kIluC][NK], r[kIluC];
+#pragma unroll
+        for (int u = 0; u < kIluC; u++) {
+#pragma unroll
+            for (int k = 0; k < NK; k++) a[u][k] = in[k * CT + u * kIluT];
+            r[u] = in[NK * CT + u * kIluT];
+        }
+        __syncwarp();
+        if (lane == 0) ilu_mbar_arrive(empty + slot);
+        ilu_mbar_wait(ffull + fslot, (unsigned)(c / kIluFaceSlots) & 1u, err, gave_up);
+#pragma unroll
+        for (int q = 0; q < kIluC; q++) {
+            const int u = FWD ? q : kIluC - 1 - q;
+            const double* fr = fring + (fslot * kIluC + u) * 32;
+            const double ny = *(edge_y ? fr + tz : sh + p * kIluT + tid + (FWD ? -1 : 1));
+            const double nz = *(edge_z ? fr + 16 + ty : sh + p * kIluT + tid + (FWD ? -kIluTY : kIluTY));
+            double aux = r[u];
+            if constexpr (FWD) {
+                aux -= a[u][0] * nz;
+                aux -= a[u][1] * ny;
+                aux -= a[u][2] * own;
+                own = aux;
+            } else {
+                aux -= a[u][0] * own;
+                aux -= a[u][1] * ny;
+                aux -= a[u][2] * nz;
+                const double q0 = aux * a[u][NK - 1];
+                own = fma(fma(-q0, a[u][NK - 2], aux), a[u][NK - 1], q0);
             }
+            sh[(p ^ 1) * kIluT + tid] = own;
+            const int step = s0 + u;
+            vt[(long long)step * kIluT] = own;
+            if (out_y) ilu_face_store(face + (long long)step * 32 + tz, own, tag);
+            if (out_z) ilu_face_store(face + (long long)step * 32 + 16 + ty, own, tag);
+            asm volatile("bar.sync 1, %0;" ::"n"(kIluT) : "memory");
+            p ^= 1;
         }
-    };
-    auto bwd_operands = [&](int level) {
-        const int s0 = start[level], cnt = start[level + 1] - s0;
-#pragma unroll
-        for (int k = 0; k < CMAX; k++) {
-            const int q = tid + k * T;
-            pos[k] = q < cnt ? s0 + q : -1;
-            if (pos[k] >= 0) {
-                const int p = pos[k];
-                v0[k] = __ldcg(yp + p);
-                v1[k] = fac[3 * n + p];
-                v2[k] = fac[4 * n + p];
-                v3[k] = fac[5 * n + p];
-                v4[k] = fac[6 * n + p];
-                n0[k] = nbr[3 * n + p];
-                n1[k] = nbr[4 * n + p];
-                n2[k] = nbr[5 * n + p];
-            }
-        }
-    };
-    unsigned int target = 0;
-    fwd_operands(0);
-    for (int level = 0; level < planes; level++) {
-#pragma unroll
-        for (int k = 0; k < CMAX; k++) {
-            if (pos[k] < 0) continue;
-            double aux = v0[k];
-            if (n0[k] >= 0) aux -= v1[k] * __ldcg(yp + n0[k]);
-            if (n1[k] >= 0) aux -= v2[k] * __ldcg(yp + n1[k]);
-            if (n2[k] >= 0) aux -= v3[k] * __ldcg(yp + n2[k]);
-            yp[pos[k]] = aux;
-        }
-        if (level + 1 < planes) fwd_operands(level + 1);
-        target += gridDim.x;
-        if (!ilu_grid_barrier(bar, target, err)) return;
-    }
-    bwd_operands(planes - 1);
-    for (int level = planes - 1; level >= 0; level--) {
-#pragma unroll
-        for (int k = 0; k < CMAX; k++) {
-            if (pos[k] < 0) continue;
-            double aux = v0[k];
-            if (n0[k] >= 0) aux -= v1[k] * __ldcg(xp + n0[k]);
-            if (n1[k] >= 0) aux -= v2[k] * __ldcg(xp + n1[k]);
-            if (n2[k] >= 0) aux -= v3[k] * __ldcg(xp + n2[k]);
-            const double v = aux / v4[k];
-            xp[pos[k]] = v;
-            x[perm[pos[k]]] = v;
-        }
-        if (level > 0) {
-            bwd_operands(level - 1);
-            target += gridDim.x;
-            if (!ilu_grid_barrier(bar, target, err)) return;
-        }
+        if (lane == 0) ilu_mbar_arrive(fempty + fslot);
     }
 }
 

@@ -227,24 +227,18 @@ struct Context {
     DevBuf<float> Z32;        // FP32 preconditioned basis (FP32 multigrid)
     DevBuf<double> gs_partial, gs_sg, gs_L;   // low-synchronisation Gram-Schmidt
     // ILU(0)
-    DevBuf<double> iluL, iluU;        // 3 lower planes (b s w) / 4 planes (p e n t), U diagonal = plane 0
+    DevBuf<double> iluL, iluU;        // 3 lower planes (b s w; natural-order sweeps only), pivots
     bool have_ilu = false;
-    // the level-scheduled ILU(0) solves as one CUDA graph (instantiated on
-    // first use, reading ilu_in and writing ilu_out)
-    cudaGraphExec_t ilu_exec = nullptr;
-    long long ilu_nodes = 0;
-    DevBuf<double> ilu_in, ilu_out;
-    // the one-launch ILU sweep (k_ilu_sweep_perm): factors, neighbour
-    // positions and work vectors in hyperplane order, the plane offsets, its
-    // barrier counter, the flag its bounded barrier sets when it gives up,
-    // its grid size and positions per thread
-    DevBuf<int> ilu_start, ilu_rowstart, ilu_perm, ilu_nbr;
-    DevBuf<double> ilu_fac, ilu_yp, ilu_xp;
-    int ilu_planes = 0, ilu_maxplane = 0;
-    DevBuf<unsigned int> ilu_bar;
-    DevBuf<int> ilu_err;
-    int ilu_blocks = 0;
-    int ilu_cmax = 0;
+    // the tiled sweeps (k_ilu_tile_sweep): geometry (nc 0: natural-order
+    // sweeps), the tiles in the order of their diagonals, coefficients, the
+    // vector and the face values in step order, the ticket counter, the flag
+    // that a wait sets when it gives up, and the sweeps launched so far
+    IluTiles ilu_g{};
+    DevBuf<int> ilu_order, ilu_err;
+    DevBuf<double> ilu_facL, ilu_facU, ilu_v;
+    DevBuf<uint4> ilu_faces;
+    DevBuf<unsigned> ilu_ticket;
+    unsigned ilu_sweeps_run = 0;
     double bytes = 0;
     int vcycles = 0;
     bool own_stream = true;
@@ -296,7 +290,6 @@ struct lsg_ctx {
 namespace lsg {
 
 static void ilu_apply(Context& C, const double* b, double* x);
-static void ilu_graph_release(Context& C);
 static void ilu_check(Context& C);
 
 // ---------------------------------------------------------------------------
@@ -1584,7 +1577,7 @@ __global__ void k_operator_grad7(int N, int M, int K, const double* __restrict__
 }
 
 // ---------------------------------------------------------------------------
-// ILU(0): pivots by hyperplane sweeps, level-scheduled solves in a CUDA graph
+// ILU(0): pivots by hyperplane sweeps, solves as a pipeline of tiles
 // ---------------------------------------------------------------------------
 
 static void ilu_setup(Context& C)
@@ -1592,184 +1585,116 @@ static void ilu_setup(Context& C)
     const Dims& d = C.d;
     LSG_REQUIRE(d.N >= 3 && d.M >= 3 && d.K >= 3, LSG_ERR_ARG, "ILU(0) needs N, M, K >= 3");
     const long long n = C.n;
-    ilu_graph_release(C);              // factors and work buffers may move
     C.iluU.alloc(n);
-    C.iluL.alloc(3 * n);
     const int planes = d.N + d.M + d.K - 2;
     const int blocks = grid_for((long long)d.N * d.M, 256);
     for (int lv = 0; lv < planes; lv++) {
         k_ilu_pivots<<<blocks, 256, 0, C.s>>>(lv, d.N, d.M, d.K, C.A7.p, C.iluU.p);
     }
     LSG_CHECK_LAUNCH();
-    k_ilu_lower<<<grid_for(n, 256), 256, 0, C.s>>>(d.N, d.M, d.K, C.A7.p, C.iluU.p, C.iluL.p);
-    LSG_CHECK_LAUNCH();
-    // the factors in hyperplane order for the one-launch sweep (grids of fewer
-    // than 2^31 cells): plane offsets and row offsets on the host, the rest
-    // on the device
-    C.ilu_blocks = 0;
-    C.ilu_planes = 0;
-    if (n < (1LL << 31) && C.s) {
-        const int P = planes, N = d.N, M = d.M, K = d.K;
-        std::vector<int> start(P + 1, 0), rowstart((size_t)P * K, 0);
-        int maxplane = 0;
-        for (int l = 0; l < P; l++) {
-            long long acc = 0;
-            for (int z = 0; z < K; z++) {
-                rowstart[(size_t)l * K + z] = (int)acc;
-                const int lz = l - z;
-                if (lz < 0) continue;
-                const int ylo = std::max(0, lz - (N - 1)), yhi = std::min(M - 1, lz);
-                if (yhi >= ylo) acc += yhi - ylo + 1;
-            }
-            start[l + 1] = start[l] + (int)acc;
-            maxplane = std::max(maxplane, (int)acc);
-        }
-        LSG_REQUIRE(start[P] == n, LSG_ERR_STATE, "hyperplane count mismatch");
-        C.ilu_planes = P;
-        C.ilu_maxplane = maxplane;
-        C.ilu_start.alloc(P + 1);
-        C.ilu_rowstart.alloc((size_t)P * K);
-        C.ilu_perm.alloc(n);
-        C.ilu_nbr.alloc(6 * (size_t)n);
-        C.ilu_fac.alloc(7 * (size_t)n);
-        C.ilu_yp.alloc(n);
-        C.ilu_xp.alloc(n);
-        LSG_CUDA(cudaMemcpyAsync(C.ilu_start.p, start.data(), start.size() * sizeof(int), cudaMemcpyHostToDevice,
+    // The tile layout pads x by 30 steps and y, z to whole tiles.  Grids that
+    // it would more than quadruple (a few cells in x, or slivers in y or z)
+    // and that hold enough for it to matter (8M positions, 0.7 GB) keep the
+    // natural order and one launch per hyperplane.
+    const IluTiles g = ilu_tiles(d.N, d.M, d.K);
+    const long long pos = g.positions(), ntile = (long long)g.nty * g.ntz;
+    C.ilu_g = (pos <= 4 * n || pos <= (8LL << 20)) ? g : IluTiles{};
+    if (C.ilu_g.nc) {
+        std::vector<int> order((size_t)ntile);
+        size_t q = 0;
+        for (int k = 0; k < g.nty + g.ntz - 1; k++)
+            for (int b = std::max(0, k - g.nty + 1); b <= std::min(k, g.ntz - 1); b++)
+                order[q++] = (k - b) + b * g.nty;
+        C.ilu_order.alloc(order.size());
+        C.ilu_facL.alloc((size_t)pos * kIluFwd);
+        C.ilu_facU.alloc((size_t)pos * kIluBwd);
+        C.ilu_v.alloc((size_t)pos);
+        C.ilu_faces.alloc((size_t)(ntile * g.steps() * 32));
+        C.ilu_ticket.alloc(1);
+        C.ilu_err.alloc(1);
+        C.ilu_sweeps_run = 0;
+        LSG_CUDA(cudaMemcpyAsync(C.ilu_order.p, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice,
                                  C.s));
-        LSG_CUDA(cudaMemcpyAsync(C.ilu_rowstart.p, rowstart.data(), rowstart.size() * sizeof(int),
-                                 cudaMemcpyHostToDevice, C.s));
-        k_ilu_perm_build<<<grid_for(n, 256), 256, 0, C.s>>>(N, M, K, C.ilu_start.p, C.ilu_rowstart.p, C.iluL.p,
-                                                            C.A7.p, C.iluU.p, C.ilu_perm.p, C.ilu_fac.p,
-                                                            C.ilu_nbr.p);
+        LSG_CUDA(cudaMemsetAsync(C.ilu_faces.p, 0, C.ilu_faces.bytes(), C.s));
+        LSG_CUDA(cudaMemsetAsync(C.ilu_ticket.p, 0, sizeof(unsigned), C.s));
+        LSG_CUDA(cudaMemsetAsync(C.ilu_err.p, 0, sizeof(int), C.s));
+        k_ilu_tile_factors<<<grid_for(pos, 256), 256, 0, C.s>>>(g, C.A7.p, C.iluU.p, C.ilu_facL.p, C.ilu_facU.p);
         LSG_CHECK_LAUNCH();
+        LSG_CUDA(cudaFuncSetAttribute(k_ilu_tile_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)ilu_sweep_smem<true>()));
+        LSG_CUDA(cudaFuncSetAttribute(k_ilu_tile_sweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)ilu_sweep_smem<false>()));
+        LSG_CUDA(cudaStreamSynchronize(C.s));     // the order table goes out of scope
+        C.iluL.release();
+        C.iluU.release();                         // the pivots are in facU
+    } else {
+        C.iluL.alloc(3 * n);
+        k_ilu_lower<<<grid_for(n, 256), 256, 0, C.s>>>(d.N, d.M, d.K, C.A7.p, C.iluU.p, C.iluL.p);
+        LSG_CHECK_LAUNCH();
+        LSG_CUDA(cudaStreamSynchronize(C.s));
     }
-    LSG_CUDA(cudaStreamSynchronize(C.s));
     C.have_ilu = true;
 }
 
-// x = U^{-1} L^{-1} b ; uses C.t4 for the intermediate
+// x = U^{-1} L^{-1} b in natural order, one launch per hyperplane; uses C.t4
+// for the intermediate
 static void ilu_sweeps(Context& C, const double* b, double* x)
 {
     const Dims& d = C.d;
     const int planes = d.N + d.M + d.K - 2;
     const int blocks = grid_for((long long)d.N * d.M, 256);
     double* y = C.t4.p;
-    for (int lv = 0; lv < planes; lv++)
+    for (int lv = 0; lv < planes; lv++) {
         k_ilu_fwd<<<blocks, 256, 0, C.s>>>(lv, d.N, d.M, d.K, C.iluL.p, b, y);
-    for (int lv = planes - 1; lv >= 0; lv--)
-        k_ilu_bwd<<<blocks, 256, 0, C.s>>>(lv, d.N, d.M, d.K, C.A7.p, C.iluU.p, y, x);
-}
-
-static void ilu_graph_release(Context& C)
-{
-    if (C.ilu_exec) cudaGraphExecDestroy(C.ilu_exec);
-    C.ilu_exec = nullptr;
-}
-
-// Both sweeps of one ILU(0) application as one cooperative launch
-// (k_ilu_sweep_perm over the hyperplane-ordered factors: a grid barrier
-// between hyperplanes instead of a kernel boundary, one launch instead of
-// 2 (N + M + K - 2)).  The grid covers the largest plane with at most a third
-// of the CTAs that fit on the GPU at once, so the three momentum equations'
-// solves still run side by side.  false = not available (the caller replays
-// the per-plane graph).
-static bool ilu_coop(Context& C, const double* b, double* x, int withhold = -1)
-{
-    if (C.ilu_blocks == 0) {
-        int dev = 0, sms = 0, coop = 0, per_sm[3] = {0, 0, 0};
-        LSG_CUDA(cudaGetDevice(&dev));
-        LSG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        LSG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        LSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[0], k_ilu_sweep_perm<1>, 256, 0));
-        LSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[1], k_ilu_sweep_perm<2>, 256, 0));
-        LSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[2], k_ilu_sweep_perm<4>, 256, 0));
-        // the fewest positions per thread (1, 2 or 4) for which the grid, as
-        // wide as the largest plane, fits a third of the CTAs the GPU holds
-        const long long cols = C.ilu_maxplane;
-        C.ilu_cmax = 0;
-        for (int q = 0; q < 3 && !C.ilu_cmax; q++) {
-            const int c = 1 << q;
-            if ((cols + 256LL * c - 1) / (256LL * c) <= (long long)sms * per_sm[q] / 3) C.ilu_cmax = c;
-        }
-        const long long need = C.ilu_cmax ? (cols + 256LL * C.ilu_cmax - 1) / (256LL * C.ilu_cmax) : 0;
-        C.ilu_blocks = (coop && C.ilu_cmax && C.ilu_planes > 0) ? (int)std::max(1LL, need) : -1;
-        if (C.ilu_blocks > 0) {
-            C.ilu_bar.alloc(1);
-            C.ilu_err.alloc(1);
-            LSG_CUDA(cudaMemsetAsync(C.ilu_err.p, 0, sizeof(int), C.s));
-        }
+        LSG_CHECK_LAUNCH();
     }
-    if (C.ilu_blocks < 0) return false;
-    LSG_CUDA(cudaMemsetAsync(C.ilu_bar.p, 0, sizeof(unsigned int), C.s));
-    int planes = C.ilu_planes;
-    long long nn = C.n;
-    const int* start = C.ilu_start.p;
-    const int* perm = C.ilu_perm.p;
-    const double* fac = C.ilu_fac.p;
-    const int* nbr = C.ilu_nbr.p;
-    double* yp = C.ilu_yp.p;
-    double* xp = C.ilu_xp.p;
-    unsigned int* bar = C.ilu_bar.p;
-    int* err = C.ilu_err.p;
-    void* args[] = {&planes, &nn, (void*)&start, (void*)&perm, (void*)&fac, (void*)&nbr, (void*)&b, &yp, &xp, &x,
-                    &bar, &err, &withhold};
-    const void* fn = C.ilu_cmax == 1   ? (const void*)k_ilu_sweep_perm<1>
-                     : C.ilu_cmax == 2 ? (const void*)k_ilu_sweep_perm<2>
-                                       : (const void*)k_ilu_sweep_perm<4>;
-    LSG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(C.ilu_blocks), dim3(256), args, 0, C.s));
-    LSG_CHECK_LAUNCH();
-    return true;
+    for (int lv = planes - 1; lv >= 0; lv--) {
+        k_ilu_bwd<<<blocks, 256, 0, C.s>>>(lv, d.N, d.M, d.K, C.A7.p, C.iluU.p, y, x);
+        LSG_CHECK_LAUNCH();
+    }
 }
 
-// Raises the failure of a cooperative ILU sweep whose barrier gave up.
+template <bool FWD>
+static void ilu_tile_sweep(Context& C, int withhold)
+{
+    const IluTiles& g = C.ilu_g;
+    const unsigned ntile = (unsigned)(g.nty * g.ntz), run = C.ilu_sweeps_run++;
+    k_ilu_tile_sweep<FWD><<<ntile, kIluThreads, ilu_sweep_smem<FWD>(), C.s>>>(
+        g, C.ilu_order.p, FWD ? C.ilu_facL.p : C.ilu_facU.p, C.ilu_v.p, C.ilu_faces.p, run + 1, C.ilu_ticket.p,
+        run * ntile, C.ilu_err.p, withhold);
+    LSG_CHECK_LAUNCH();
+}
+
+// x = U^{-1} L^{-1} b: b into the tiles' order, the two sweeps in place, back.
+static void ilu_tiles_apply(Context& C, const double* b, double* x, int withhold = -1)
+{
+    const IluTiles& g = C.ilu_g;
+    const dim3 vg((unsigned)(g.nty * g.ntz), (unsigned)((g.steps() + 31) / 32), 4);
+    k_ilu_tile_vector<true><<<vg, 256, 0, C.s>>>(g, b, C.ilu_v.p);
+    LSG_CHECK_LAUNCH();
+    ilu_tile_sweep<true>(C, withhold);
+    ilu_tile_sweep<false>(C, -1);
+    k_ilu_tile_vector<false><<<vg, 256, 0, C.s>>>(g, C.ilu_v.p, x);
+    LSG_CHECK_LAUNCH();
+}
+
+// Raises the failure of a sweep in which a wait gave up.
 static void ilu_check(Context& C)
 {
-    if (C.opt.precond != LSG_PC_ILU0 || C.ilu_blocks <= 0) return;
+    if (C.opt.precond != LSG_PC_ILU0 || !C.ilu_g.nc) return;
     int e = 0;
     LSG_CUDA(cudaMemcpyAsync(&e, C.ilu_err.p, sizeof(int), cudaMemcpyDeviceToHost, C.s));
     LSG_CUDA(cudaStreamSynchronize(C.s));
     if (e) {
         LSG_CUDA(cudaMemsetAsync(C.ilu_err.p, 0, sizeof(int), C.s));
-        throw Error{LSG_ERR_CUDA, "an ILU sweep's grid barrier gave up waiting"};
+        throw Error{LSG_ERR_CUDA, "an ILU sweep's wait at a tile barrier gave up"};
     }
 }
 
-// The 2 (N + M + K - 2) hyperplane launches of one application are replayed
-// as one CUDA graph: b is copied into a fixed input buffer, the graph runs,
-// the result is copied out (two device copies of n values against hundreds
-// of launch submissions).  A context on the legacy default stream launches
-// the sweeps directly.
 static void ilu_apply(Context& C, const double* b, double* x)
 {
-    if (!C.s) {
-        ilu_sweeps(C, b, x);
-        LSG_CHECK_LAUNCH();
-        return;
-    }
-    if (ilu_coop(C, b, x)) return;
-    const long long n = C.n;
-    if (!C.ilu_exec) {
-        C.ilu_in.alloc(n);
-        C.ilu_out.alloc(n);
-        cudaGraph_t graph = nullptr;
-        LSG_CUDA(cudaStreamBeginCapture(C.s, cudaStreamCaptureModeThreadLocal));
-        ilu_sweeps(C, C.ilu_in.p, C.ilu_out.p);
-        const cudaError_t launch_err = cudaGetLastError();
-        const cudaError_t cap_err = cudaStreamEndCapture(C.s, &graph);
-        LSG_CUDA(launch_err);
-        LSG_CUDA(cap_err);
-        size_t nodes = 0;
-        cudaGraphGetNodes(graph, nullptr, &nodes);
-        C.ilu_nodes = (long long)nodes;
-        const cudaError_t inst_err = cudaGraphInstantiate(&C.ilu_exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (inst_err != cudaSuccess) C.ilu_exec = nullptr;
-        LSG_CUDA(inst_err);
-    }
-    LSG_CUDA(cudaMemcpyAsync(C.ilu_in.p, b, n * sizeof(double), cudaMemcpyDeviceToDevice, C.s));
-    LSG_CUDA(cudaGraphLaunch(C.ilu_exec, C.s));
-    ::lsg::g_launches += C.ilu_nodes;
-    LSG_CUDA(cudaMemcpyAsync(x, C.ilu_out.p, n * sizeof(double), cudaMemcpyDeviceToDevice, C.s));
+    if (C.ilu_g.nc) ilu_tiles_apply(C, b, x);
+    else ilu_sweeps(C, b, x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1945,7 +1870,6 @@ static cudaStream_t context_release(Context& C)
         C.adj.reset();
     }
     if (C.s) cudaStreamSynchronize(C.s);
-    ilu_graph_release(C);
     vcycle_graphs_release(C.mg);
     if (C.hflag) cudaFreeHost(C.hflag);
     C.hflag = nullptr;
@@ -3183,7 +3107,6 @@ int lsg_setup(lsg_ctx* h, const lsg_options* opts)
     WallTimer wt(C.setup_ms);
     LSG_REQUIRE(C.have_matrix, LSG_ERR_STATE, "lsg_set_matrix_csr must be called before lsg_setup");
     LSG_CUDA(cudaSetDevice(C.device));
-    ilu_graph_release(C);                  // work buffers are (re)allocated below
     if (opts) C.opt = *opts;
     LSG_REQUIRE(C.opt.method == LSG_METHOD_FGMRES || C.opt.method == LSG_METHOD_BICGSTAB, LSG_ERR_ARG, "bad method");
     LSG_REQUIRE(C.opt.precond >= 0 && C.opt.precond <= 2, LSG_ERR_ARG, "bad preconditioner");
@@ -3842,10 +3765,8 @@ int lsg_selftest_wait_limit(lsg_ctx* h)
     LSG_REQUIRE(C.have_setup && C.opt.precond == LSG_PC_ILU0, LSG_ERR_STATE, "needs lsg_setup with ILU(0)");
     LSG_CUDA(cudaSetDevice(C.device));
     LSG_CUDA(cudaMemsetAsync(C.t1.p, 0, C.n * sizeof(double), C.s));
-    if (C.ilu_blocks == 0) ilu_coop(C, C.t1.p, C.t2.p);   // sizes the sweep (a normal run)
-    LSG_REQUIRE(C.ilu_blocks >= 2, LSG_ERR_STATE, "the self-test needs a one-launch sweep of two CTAs or more");
-    LSG_CUDA(cudaStreamSynchronize(C.s));
-    ilu_coop(C, C.t1.p, C.t2.p, 0);                // CTA 0 withholds its first arrival
+    LSG_REQUIRE(C.ilu_g.nty * C.ilu_g.ntz >= 2, LSG_ERR_STATE, "the self-test needs a sweep of two tiles or more");
+    ilu_tiles_apply(C, C.t1.p, C.t2.p, 0);         // the first tile's CTA writes no face
     ilu_check(C);                                  // throws: the others' wait ran out
     return LSG_OK;
     LSG_API_END(h)
