@@ -150,6 +150,14 @@ __global__ void k_ilu_bwd(int level, int N, int M, int K, const double* __restri
 // memory), and a step costs one barrier of one CTA.  Only the tile's two
 // faces are exchanged between CTAs.
 //
+// Bound by the chain of dependent steps, N + M + K - 2 of them and the hand-over
+// at each tile border, until a grid has enough tiles to fill the memory pipe.
+// 16 x 16 lines keep the border crossings few (M/16 + K/16) with a barrier over
+// only eight warps.  Measured on a B200, a momentum solve of 127 x 64 x 64 (two
+// iterations): 0.56 ms against 2.30 ms with one cooperative launch and a grid
+// barrier per hyperplane; an ILU-BiCGStab solve of 64 x 48 x 40: 35 against
+// 139 ms.  The same bits.
+//
 // Storage follows the steps: position (tile, step, thread), so that every
 // stream is contiguous in the order in which it is used.  A tile has
 // S = N + 30 steps, rounded up to whole chunks of kIluC; positions outside
