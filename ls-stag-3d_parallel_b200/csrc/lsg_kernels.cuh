@@ -222,72 +222,6 @@ __global__ void __launch_bounds__(256) k_apply7(int N, int M, int K, const T* __
     }
 }
 
-// Box-stencil (coarse Galerkin operator) residual update r -= A x (mode 0)
-// or y = A x (mode 1).
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256) k_applybox(int N, int M, int K, OffList ol, const T* __restrict__ coef,
-                                                   const T* __restrict__ x, T* __restrict__ r)
-{
-    const long long n = (long long)N * M * K;
-    const int NM = N * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int ix, iy, iz;
-        cell_xyz(i, N, NM, ix, iy, iz);
-        T acc = 0;
-        for (int o = 0; o < ol.n; o++) {
-            const int jx = ix + ol.o[o][0], jy = iy + ol.o[o][1], jz = iz + ol.o[o][2];
-            if (jx < 0 || jx >= N || jy < 0 || jy >= M || jz < 0 || jz >= K) continue;
-            acc += coef[(size_t)o * n + i] * x[i + ol.o[o][0] + (long long)ol.o[o][1] * N + (long long)ol.o[o][2] * NM];
-        }
-        if (MODE == 0) r[i] -= acc;
-        else r[i] = acc;
-    }
-}
-
-// 27-point box stencil (radius 1 in every dimension, the Galerkin operator of
-// the even-even-even and odd-odd-odd coarsenings): offsets unrolled, plane
-// q = ((dz+1)*3 + (dy+1))*3 + (dx+1).
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256) k_apply27(int N, int M, int K, const T* __restrict__ coef,
-                                                  const T* __restrict__ x, T* __restrict__ r)
-{
-    const long long n = (long long)N * M * K;
-    const int NM = N * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int ix, iy, iz;
-        cell_xyz(i, N, NM, ix, iy, iz);
-        T acc = 0;
-        const bool interior = ix > 0 && ix < N - 1 && iy > 0 && iy < M - 1 && iz > 0 && iz < K - 1;
-        if (interior) {
-#pragma unroll
-            for (int dz = -1; dz <= 1; dz++)
-#pragma unroll
-                for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-                    for (int dx = -1; dx <= 1; dx++) {
-                        const int q = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
-                        acc += coef[(size_t)q * n + i] * x[i + dx + (long long)dy * N + (long long)dz * NM];
-                    }
-        } else {
-#pragma unroll
-            for (int dz = -1; dz <= 1; dz++)
-#pragma unroll
-                for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-                    for (int dx = -1; dx <= 1; dx++) {
-                        const int jx = ix + dx, jy = iy + dy, jz = iz + dz;
-                        if (jx < 0 || jx >= N || jy < 0 || jy >= M || jz < 0 || jz >= K) continue;
-                        const int q = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
-                        acc += coef[(size_t)q * n + i] * x[i + dx + (long long)dy * N + (long long)dz * NM];
-                    }
-        }
-        if (MODE == 0) r[i] -= acc;
-        else r[i] = acc;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // row-dictionary operators: cls[i] indexes a table of the distinct
 // coefficient rows (row-major, NOFF values per row).  Bit-identical rows share
@@ -313,48 +247,6 @@ __global__ void __launch_bounds__(256) k_apply7d(int N, int M, int K, const int*
         if (ix < N - 1) acc += a[4] * x[i + 1];
         if (iy < M - 1) acc += a[5] * x[i + N];
         if (iz < K - 1) acc += a[6] * x[i + NM];
-        if (MODE == 0) r[i] -= acc;
-        else r[i] = acc;
-    }
-}
-
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256) k_apply27d(int N, int M, int K, const int* __restrict__ cls,
-                                                   const T* __restrict__ dict, const T* __restrict__ x,
-                                                   T* __restrict__ r)
-{
-    const long long n = (long long)N * M * K;
-    const int NM = N * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int ix, iy, iz;
-        cell_xyz(i, N, NM, ix, iy, iz);
-        const T* a = dict + (size_t)cls[i] * 27;
-        T acc = 0;
-        const bool interior = ix > 0 && ix < N - 1 && iy > 0 && iy < M - 1 && iz > 0 && iz < K - 1;
-        if (interior) {
-#pragma unroll
-            for (int dz = -1; dz <= 1; dz++)
-#pragma unroll
-                for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-                    for (int dx = -1; dx <= 1; dx++) {
-                        const int q = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
-                        acc += a[q] * x[i + dx + (long long)dy * N + (long long)dz * NM];
-                    }
-        } else {
-#pragma unroll
-            for (int dz = -1; dz <= 1; dz++)
-#pragma unroll
-                for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-                    for (int dx = -1; dx <= 1; dx++) {
-                        const int jx = ix + dx, jy = iy + dy, jz = iz + dz;
-                        if (jx < 0 || jx >= N || jy < 0 || jy >= M || jz < 0 || jz >= K) continue;
-                        const int q = ((dz + 1) * 3 + (dy + 1)) * 3 + (dx + 1);
-                        acc += a[q] * x[i + dx + (long long)dy * N + (long long)dz * NM];
-                    }
-        }
         if (MODE == 0) r[i] -= acc;
         else r[i] = acc;
     }
@@ -531,27 +423,83 @@ __global__ void k_pad_rows(long long nrows, int w, int wpad, const double* __res
     }
 }
 
-template <typename T, int MODE>
-__global__ void __launch_bounds__(256) k_applyboxd(int N, int M, int K, OffList ol, const int* __restrict__ cls,
-                                                    const T* __restrict__ dict, const T* __restrict__ x,
-                                                    T* __restrict__ r)
+// Box stencils wider than 27 points (levels below a coarsening of mixed
+// parity): radius R* per dimension, offsets in z, y, x order.  One thread per
+// cell with the loops unrolled, so the row and the neighbours are all in
+// flight; a generic loop over an offset list waited for each coefficient in
+// turn.  Latency bound on these levels: the loop took 30 us a launch on the
+// levels of a 150 x 90 x 70 hierarchy, the two forms here 4.5; its FP64 solve
+// 14.9 -> 7.8 ms, that of 32 x 24 x 20 4.66 -> 3.27 ms.
+template <typename T, int MODE, int RX, int RY, int RZ>
+__global__ void __launch_bounds__(128) k_applybox(int N, int M, int K, const int* __restrict__ cls,
+                                                   const T* __restrict__ dict, const T* __restrict__ x,
+                                                   T* __restrict__ r)
 {
-    const long long n = (long long)N * M * K;
-    const int NM = N * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        int ix, iy, iz;
-        cell_xyz(i, N, NM, ix, iy, iz);
-        const T* a = dict + (size_t)cls[i] * ol.n;
+    constexpr int BX = 2 * RX + 1, BY = 2 * RY + 1, BZ = 2 * RZ + 1;
+    const int ix = blockIdx.x * 32 + threadIdx.x;
+    const int iy = blockIdx.y * 4 + threadIdx.y;
+    if (ix >= N || iy >= M) return;
+    const int NM = N * M;                                  // grids hold fewer than 2^31 cells
+    for (int iz = blockIdx.z; iz < K; iz += gridDim.z) {
+        const int i = ix + N * iy + NM * iz;
+        const T* a = dict + (size_t)cls[i] * (BX * BY * BZ);
+        const T old = MODE == 0 ? r[i] : (T)0;
         T acc = 0;
-        for (int o = 0; o < ol.n; o++) {
-            const int jx = ix + ol.o[o][0], jy = iy + ol.o[o][1], jz = iz + ol.o[o][2];
-            if (jx < 0 || jx >= N || jy < 0 || jy >= M || jz < 0 || jz >= K) continue;
-            acc += a[o] * x[i + ol.o[o][0] + (long long)ol.o[o][1] * N + (long long)ol.o[o][2] * NM];
-        }
-        if (MODE == 0) r[i] -= acc;
-        else r[i] = acc;
+#pragma unroll
+        for (int dz = -RZ; dz <= RZ; dz++)
+#pragma unroll
+            for (int dy = -RY; dy <= RY; dy++) {
+                const bool row = iz + dz >= 0 && iz + dz < K && iy + dy >= 0 && iy + dy < M;
+                const T* xr = x + i + dz * NM + dy * N;
+                T v[BX], c[BX];
+#pragma unroll
+                for (int dx = -RX; dx <= RX; dx++) {
+                    const bool ok = row && ix + dx >= 0 && ix + dx < N;
+                    v[dx + RX] = ok ? xr[dx] : (T)0;
+                    c[dx + RX] = a[((dz + RZ) * BY + dy + RY) * BX + dx + RX];
+                }
+#pragma unroll
+                for (int k = 0; k < BX; k++) acc += c[k] * v[k];
+            }
+        r[i] = MODE == 0 ? old - acc : acc;
     }
+}
+
+// The same on small levels, where one thread per cell leaves the GPU idle and
+// each thread waits for its own distinct row: eight lanes per cell, the row
+// read side by side, the partial sums added by shuffles.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(128) k_applybox8(int N, int M, int K, int rx, int ry, int rz,
+                                                    const int* __restrict__ cls, const T* __restrict__ dict,
+                                                    const T* __restrict__ x, T* __restrict__ r)
+{
+    const int bx = 2 * rx + 1, by = 2 * ry + 1, nb = bx * by * (2 * rz + 1);
+    const int NM = N * M, n = NM * K;                      // small levels: int
+    __shared__ int so[128][4];                             // dx, dy, dz, flat offset (nb <= 125)
+    if (threadIdx.x < nb) {
+        const int o = threadIdx.x, dz = o / (bx * by) - rz, dy = (o / bx) % by - ry, dx = o % bx - rx;
+        so[o][0] = dx;
+        so[o][1] = dy;
+        so[o][2] = dz;
+        so[o][3] = dx + dy * N + dz * NM;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 7;
+    const int i = blockIdx.x * 16 + (threadIdx.x >> 3);
+    const bool in = i < n;
+    const int q = in ? i : n - 1;
+    const int z = q / NM, rem = q - z * NM, y = rem / N, xx = rem - y * N;
+    const T* a = dict + (size_t)cls[q] * nb;
+    T acc = 0;
+#pragma unroll 4
+    for (int o = lane; o < nb; o += 8) {
+        const int jx = xx + so[o][0], jy = y + so[o][1], jz = z + so[o][2];
+        const bool ok = jx >= 0 && jx < N && jy >= 0 && jy < M && jz >= 0 && jz < K;
+        acc += a[o] * (ok ? x[q + so[o][3]] : (T)0);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, 8);
+    if (in && lane == 0) r[i] = MODE == 0 ? r[i] - acc : acc;
 }
 
 // ---------------------------------------------------------------------------

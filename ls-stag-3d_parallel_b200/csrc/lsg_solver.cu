@@ -820,6 +820,36 @@ static void mg_setup(Context& C)
 // V-cycle (MultiGridSolver::solve, multigrid_solver.h:48-75).
 // Input: right-hand side already in lev[0].r.  Output: lev[0].ch.
 // ---------------------------------------------------------------------------
+// Box stencils of other radii than 1, 1, 1 (each is 1 or 2; offsets in z, y,
+// x order as mg_setup lists them).  Below 32768 cells the lanes-per-cell form.
+template <typename T, int MODE>
+static void apply_box(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s)
+{
+    const Dims& d = lv.d;
+    const long long n = d.n();
+    const int rx = -lv.off[0], ry = -lv.off[1], rz = -lv.off[2];   // the first offset is the box's corner
+    LSG_REQUIRE(rx >= 1 && rx <= 2 && ry >= 1 && ry <= 2 && rz >= 1 && rz <= 2 &&
+                    lv.ol.n == (2 * rx + 1) * (2 * ry + 1) * (2 * rz + 1),
+                LSG_ERR_STATE, "unexpected coarse stencil");
+    if (n < 32768) {
+        k_applybox8<T, MODE><<<(unsigned)((n + 15) / 16), 128, 0, s>>>(d.N, d.M, d.K, rx, ry, rz, lv.cls, lv.dict, x,
+                                                                      r);
+        return;
+    }
+    const dim3 b(32, 4), g((d.N + 31) / 32, (d.M + 3) / 4, std::min(d.K, 65535));
+    auto go = [&](auto kernel) { kernel<<<g, b, 0, s>>>(d.N, d.M, d.K, lv.cls, lv.dict, x, r); };
+    switch (rx * 4 + ry * 2 + rz - 7) {
+    case 0: go(k_applybox<T, MODE, 1, 1, 1>); break;
+    case 1: go(k_applybox<T, MODE, 1, 1, 2>); break;
+    case 2: go(k_applybox<T, MODE, 1, 2, 1>); break;
+    case 3: go(k_applybox<T, MODE, 1, 2, 2>); break;
+    case 4: go(k_applybox<T, MODE, 2, 1, 1>); break;
+    case 5: go(k_applybox<T, MODE, 2, 1, 2>); break;
+    case 6: go(k_applybox<T, MODE, 2, 2, 1>); break;
+    default: go(k_applybox<T, MODE, 2, 2, 2>); break;
+    }
+}
+
 template <typename T>
 static void apply_resid(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s, int mode, int zc27 = 0)
 {
@@ -839,11 +869,10 @@ static void apply_resid(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s, i
             k_apply27z<T, 0><<<zg, zb, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
         else
             k_apply27z<T, 1><<<zg, zb, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
+    } else if (mode == 0) {
+        apply_box<T, 0>(lv, x, r, s);
     } else {
-        if (mode == 0)
-            k_applyboxd<T, 0><<<grid_for(n, 256), 256, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, lv.ol, lv.cls, lv.dict, x, r);
-        else
-            k_applyboxd<T, 1><<<grid_for(n, 256), 256, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, lv.ol, lv.cls, lv.dict, x, r);
+        apply_box<T, 1>(lv, x, r, s);
     }
     LSG_CHECK_LAUNCH();
 }
