@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256) k_mgs_step(long long n, const double* __r
 }
 
 // v = w / ||w||  (copyTo(curV, normW), mesh_function.h:256-260) and the
-// preconditioner right-hand side in its precision.
+// preconditioner right-hand side in its precision (null: it reads v).
 template <typename T>
 __global__ void k_scale_copy(long long n, const double* __restrict__ w, const double* __restrict__ invnorm,
                              double* __restrict__ v, T* __restrict__ rhs)
@@ -262,7 +262,7 @@ __global__ void k_scale_copy(long long n, const double* __restrict__ w, const do
          i += (long long)gridDim.x * blockDim.x) {
         const double t = w[i] * s;
         v[i] = t;
-        rhs[i] = (T)t;
+        if (rhs) rhs[i] = (T)t;
     }
 }
 

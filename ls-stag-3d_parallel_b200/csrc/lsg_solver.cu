@@ -1162,10 +1162,22 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
     C.vcycles++;
 }
 
-// ch0: where the finest-level correction (the preconditioned vector) goes;
-// nullptr = the level's own buffer.
+// Whether a level runs the fused ADLJ steps on these buffers (16-byte vectors
+// along x).
 template <typename T>
-static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr)
+static bool level_fused(const Context& C, const LevelT<T>& lv, const T* ch)
+{
+    const bool aligned = ((reinterpret_cast<uintptr_t>(ch) | reinterpret_cast<uintptr_t>(lv.c.p) |
+                           reinterpret_cast<uintptr_t>(lv.r.p) | reinterpret_cast<uintptr_t>(lv.cls)) & 15) == 0;
+    return C.opt.n_post > 0 && aligned && adlj_fused_level<T>(lv.d, lv.ol.n, lv.off, C.opt);
+}
+
+// ch0: where the finest-level correction (the preconditioned vector) goes;
+// nullptr = the level's own buffer.  hold_last: a fused finest level stops
+// before its last direction step, which the caller launches from the level's
+// c into the buffer it wants the correction in.
+template <typename T>
+static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr, bool hold_last = false)
 {
     if (C.opt.smoother == LSG_SMOOTHER_RBGS) {
         vcycle_rb<T>(C, lev, ch0);
@@ -1200,9 +1212,7 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr)
         T* chl = (l == 0 && ch0) ? ch0 : lv.ch.p;
         const int order[3] = {2, 1, 0};           // SmootherADLJ::solve: z, y, x
         const int steps = 3 * C.opt.n_post;
-        const bool aligned = ((reinterpret_cast<uintptr_t>(chl) | reinterpret_cast<uintptr_t>(lv.c.p) |
-                               reinterpret_cast<uintptr_t>(lv.r.p) | reinterpret_cast<uintptr_t>(lv.cls)) & 15) == 0;
-        const bool fused = steps > 0 && aligned && adlj_fused_level<T>(f, lv.ol.n, lv.off, C.opt);
+        const bool fused = level_fused<T>(C, lv, chl);
         // the fused steps alternate the iterate between c and chl, starting from
         // the buffer that makes the last step write chl: the prolongation fills
         // that one only; the reference schedule needs P c_H in both
@@ -1220,6 +1230,7 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr)
         if (fused) {
             for (int it = 0; it < C.opt.n_post; it++)
                 for (int q = 0; q < 3; q++) {
+                    if (l == 0 && hold_last && it == C.opt.n_post - 1 && q == 2) break;
                     adlj_fused_step<T>(lv, order[q], zq, omega, s, buf[cur], buf[cur ^ 1]);
                     cur ^= 1;
                 }
@@ -1241,26 +1252,30 @@ static void vcycle_graphs_release(MGData& mg)
     mg.cycle64 = mg.cycle32 = nullptr;
 }
 
-// One ADLJ V-cycle replayed from a CUDA graph: the cycle's launches (about 20
-// per level above the tail kernel) only touch the hierarchy's own buffers, so
-// they are captured once and submitted as one unit, which removes the host
-// submission gaps of the small coarse-level kernels.  The correction is left
-// in level 0's ch; ch0 (if given) receives a copy.  Contexts on the legacy
-// default stream and the Gauss-Seidel cycle run the launches directly.
+// One V-cycle replayed from a CUDA graph: the cycle's launches (about 20 per
+// level above the tail kernel, 40 with the Gauss-Seidel smoother) only touch
+// the hierarchy's own buffers, so they are captured once and submitted as one
+// unit, which removes the host submission gaps of the small coarse-level
+// kernels (a 128^3 Gauss-Seidel solve spent 7 of its 17 ms in them).  The
+// correction goes to level 0's ch, or to ch0 if given: where the finest level
+// is smoothed by the fused steps, the last of them is launched after the graph
+// and writes there itself, otherwise it is copied.  Contexts on the legacy
+// default stream run the launches directly.
 template <typename T>
 static void vcycle_run(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
 {
-    if (!C.s || C.opt.smoother == LSG_SMOOTHER_RBGS) {
+    if (!C.s) {
         vcycle<T>(C, lev, ch0);
         return;
     }
+    const bool hold = C.opt.smoother == LSG_SMOOTHER_ADLJ && level_fused<T>(C, lev[0], lev[0].ch.p);
     cudaGraphExec_t& exec = sizeof(T) == 8 ? C.mg.cycle64 : C.mg.cycle32;
     if (!exec) {
         cudaGraph_t graph = nullptr;
         LSG_CUDA(cudaStreamBeginCapture(C.s, cudaStreamCaptureModeThreadLocal));
         Error captured{LSG_OK, ""};
         try {
-            vcycle<T>(C, lev, nullptr);
+            vcycle<T>(C, lev, nullptr, hold);
         } catch (const Error& e) {
             captured = e;
         }
@@ -1283,6 +1298,12 @@ static void vcycle_run(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
     // launch accounting counts the kernels the replay runs
     ::lsg::g_launches += sizeof(T) == 8 ? C.mg.cycle64_nodes : C.mg.cycle32_nodes;
     C.vcycles++;
+    if (hold) {
+        const bool direct = ch0 && level_fused<T>(C, lev[0], ch0);
+        adlj_fused_step<T>(lev[0], 0, C.opt.zline_reference != 0, (T)C.opt.omega, C.s, lev[0].c.p,
+                           direct ? ch0 : lev[0].ch.p);
+        if (direct) return;
+    }
     if (ch0)
         LSG_CUDA(cudaMemcpyAsync(ch0, lev[0].ch.p, (size_t)lev[0].d.n() * sizeof(T), cudaMemcpyDeviceToDevice, C.s));
 }
@@ -1347,8 +1368,7 @@ static void precond_apply(Context& C, const double* v, double* z)
     } else {
         auto& lev = C.mg.l64;
         LSG_CUDA(cudaMemcpyAsync(lev[0].r.p, v, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-        vcycle_run<double>(C, lev, nullptr);
-        LSG_CUDA(cudaMemcpyAsync(z, lev[0].ch.p, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+        vcycle_run<double>(C, lev, z);
     }
 }
 
@@ -1457,11 +1477,17 @@ static int fgmres(Context& C, double* x, const double* b, lsg_stats* st)
                     LSG_CHECK_LAUNCH();
                     vcycle_run<float>(C, C.mg.l32, zj32);
                     bytes += (8 + 8 + 4) * (double)n + vcycle_bytes(C.mg, C.opt, 4.0);
-                } else {
-                    k_scale_copy<double><<<grid_for(n, 256), 256, 0, s>>>(n, C.w.p, &ks->invNormW, vj, C.t1.p);
+                } else if (C.opt.precond == LSG_PC_MG) {
+                    // straight into the cycle's right-hand side, and z_j straight out of it
+                    k_scale_copy<double><<<grid_for(n, 256), 256, 0, s>>>(n, C.w.p, &ks->invNormW, vj, C.mg.l64[0].r.p);
                     LSG_CHECK_LAUNCH();
-                    precond_apply(C, C.t1.p, zj);
-                    bytes += 24.0 * n + (C.opt.precond == LSG_PC_MG ? vcycle_bytes(C.mg, C.opt, 8.0) + 32.0 * n : 0);
+                    vcycle_run<double>(C, C.mg.l64, zj);
+                    bytes += 24.0 * n + vcycle_bytes(C.mg, C.opt, 8.0);
+                } else {
+                    k_scale_copy<double><<<grid_for(n, 256), 256, 0, s>>>(n, C.w.p, &ks->invNormW, vj, nullptr);
+                    LSG_CHECK_LAUNCH();
+                    precond_apply(C, vj, zj);
+                    bytes += 16.0 * n;
                 }
                 // w = A z_j ; H[0,j] = (w, v_0)
                 double* Hj = ks->H + (size_t)j * 65;
