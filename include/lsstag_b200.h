@@ -61,7 +61,7 @@ extern "C" {
 /* lsg_options.smoother */
 #define LSG_SMOOTHER_ADLJ 0   /* reference: damped z,y,x line Jacobi */
 #define LSG_SMOOTHER_RBGS 1   /* red-black point Gauss-Seidel (new variant) */
-#define LSG_ADLJ_AUTO 0       /* fused for the FP32 cycle, the reference's schedule for the FP64 cycle */
+#define LSG_ADLJ_AUTO 0       /* fused wherever a level's shape has the kernels */
 #define LSG_ADLJ_REFERENCE 1  /* the reference's schedule: r -= A c, then the line solve */
 #define LSG_ADLJ_FUSED 2      /* ADLJ direction step as one kernel (residual formed in the line solve) */
 
@@ -92,8 +92,7 @@ typedef struct lsg_options {
                             (smoother_adlj_interface.h:66-77) everywhere.  The
                             two are equal in exact arithmetic (r = b - A ch
                             before every direction) and differ by rounding.
-                            LSG_ADLJ_AUTO (default): fused in the FP32 cycle,
-                            the reference's schedule in the FP64 cycle. */
+                            LSG_ADLJ_AUTO (default): as LSG_ADLJ_FUSED. */
     int reserved[6];
 } lsg_options;
 
@@ -555,8 +554,8 @@ int lsg_mg_level_tridiag(lsg_ctx* ctx, int level, char dir, double* c, double* d
    solve uses on wide grids, 8 the same product by the register z-marching
    kernel (no staging; for comparison), 9/10/11 the fused ADLJ direction
    step (residual formed inside the line solve) along x/y/z on the finest
-   level (needs a level that runs it: LSG_ADLJ_FUSED, or LSG_ADLJ_AUTO in
-   FP32), 12/13 the y/z steps with the segment maps walked by each thread
+   level (needs a level that runs it: LSG_ADLJ_FUSED or LSG_ADLJ_AUTO),
+   12/13 the y/z steps with the segment maps walked by each thread
    instead of composed by log-step scans, 14/15 the same for the y/z line
    solves of the reference schedule, 16/17 those line solves with 4-cell
    segments (the FP64 z-line solve's own form), 18/19 the first coarse
