@@ -489,8 +489,6 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
             for (int k = 0; k < NK; k++) a[u][k] = in[k * CT + u * kIluT];
             r[u] = in[NK * CT + u * kIluT];
         }
-        __syncwarp();
-        if (lane == 0) ilu_mbar_arrive(empty + slot);
         ilu_mbar_wait(ffull + fslot, (unsigned)(c / kIluFaceSlots) & 1u, err, gave_up);
 #pragma unroll
         for (int q = 0; q < kIluC; q++) {
@@ -519,7 +517,13 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
             asm volatile("bar.sync 1, %0;" ::"n"(kIluT) : "memory");
             p ^= 1;
         }
-        if (lane == 0) ilu_mbar_arrive(fempty + fslot);
+        // this chunk's slots are free: its operands have been used, not only
+        // asked for (an arrival may overtake shared loads in flight, and the
+        // next copy into the slot would reach them)
+        if (lane == 0) {
+            ilu_mbar_arrive(fempty + fslot);
+            ilu_mbar_arrive(empty + slot);
+        }
     }
 }
 

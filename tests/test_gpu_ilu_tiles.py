@@ -63,3 +63,47 @@ def test_thin_grid_keeps_the_natural_order():
     s.close()
     # a backward-stable tridiagonal solve: a few units of 1e-16 times |A||x|
     assert np.abs(r).max() <= 1e-13 * np.abs(x).max()
+
+
+def test_concurrent_contexts_give_the_same_bits():
+    """Three contexts whose sweeps together have more tiles than the GPU has
+    SMs, solving at once: every solve gives the bits of a solve alone (a ring
+    slot released while its loads were in flight gave other values in one
+    solve of fifty)."""
+    import ctypes as C
+    import threading
+
+    import torch
+    from lsstag_b200 import solver as S
+    dims = (96, 128, 128)
+    P = _planes(dims, 11)
+    ctx = []
+    for k in range(3):
+        s = S.ILUFGMRES()
+        s.set_planes(P, dims, S.Task(eps=0.0, MAX_ITER=4))
+        b = torch.as_tensor(np.random.default_rng(k).standard_normal(P.shape[1]), device="cuda")
+        ctx.append((s, b, torch.empty_like(b)))
+
+    def solve(k):
+        s, b, x = ctx[k]
+        x.zero_()
+        torch.cuda.current_stream().synchronize()
+        s.ctx.check(s.ctx.lib.lsg_solve_device(s.ctx.h, C.c_void_p(b.data_ptr()), C.c_void_p(x.data_ptr()),
+                                               C.byref(s.stats)))
+        return x
+
+    want = [solve(k).clone() for k in range(3)]
+    differ = [0, 0, 0]
+
+    def many(k):
+        for _ in range(120):
+            differ[k] += not torch.equal(solve(k), want[k])
+
+    threads = [threading.Thread(target=many, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for s, _, _ in ctx:
+        s.close()
+    assert differ == [0, 0, 0]
