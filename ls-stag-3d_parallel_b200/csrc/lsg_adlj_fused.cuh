@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256) k_adlj_fused_xseg(int N, int M, int K, in
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        if (o >= P) break;
+        if (o >= P || !__any_sync(0xffffffffu, scan_more(fb))) break;
         const T a2 = __shfl_up_sync(0xffffffffu, fa, o, P);
         const T b2 = __shfl_up_sync(0xffffffffu, fb, o, P);
         if (q >= o) {
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256) k_adlj_fused_xseg(int N, int M, int K, in
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        if (o >= P) break;
+        if (o >= P || !__any_sync(0xffffffffu, scan_more(hh))) break;
         const T g2 = __shfl_down_sync(0xffffffffu, g, o, P);
         const T h2 = __shfl_down_sync(0xffffffffu, hh, o, P);
         if (q + o < P) {
