@@ -70,7 +70,8 @@ __device__ __forceinline__ T resid7_at(int N, int M, int K, long long q, const i
 // segments: by log-step scans in shared memory when VAR & 1 (the solve's
 // form), else by each thread walking the maps before its own (timing
 // comparison).  VAR & 2: the line splits into whole segments (L = S SEG),
-// so no cell lies past its end and the line-end guards go.  zquirk (DIR 2):
+// so no cell lies past its end and the line-end guards go.  VAR & 4: warps
+// whose cells share one row take a path of their own.  zquirk (DIR 2):
 // the first right-hand side of the z-line
 // (x, y) is the residual at cell y*N*K + x, where the reference reads it
 // (smoother_adlj_z.h:54-58).  Shared memory: 4 W S values.
@@ -119,44 +120,74 @@ __global__ void __launch_bounds__(MAXT, MINB)
     }
     const T xprev = t0 > 0 ? xin[i0 + (t0 - 1) * st] : (T)0;
     const T xnext = t0 + SEG < L ? xin[i0 + (t0 + SEG) * st] : (T)0;
-    // phase 2: residuals; lv <- lower coupling, uv <- scaled upper coupling
+    // phase 2: residuals; lv <- lower coupling, uv <- scaled upper coupling.
+    // Away from bodies and walls all cells of a warp have one row: it is read
+    // once, and no cell's neighbours need a bounds test (VAR & 4).
+    constexpr bool ONEROW = (VAR & 4) != 0;
     T lv[SEG], uv[SEG];
+    bool same = ONEROW && hw && he && hm && hp && t0 > 0 && t0 + SEG < L;
+    const unsigned lanes = __activemask();                 // all of them, or the CTA's last half warp
+    const int c0 = __shfl_sync(lanes, cl[0], 0);
 #pragma unroll
-    for (int u = 0; u < SEG; u++) {
-        const int t = t0 + u;
-        lv[u] = 0;
-        uv[u] = 0;
-        if (EXACT || t < L) {
-            const int i = i0 + t * st;
-            const T* a = dict + (size_t)cl[u] * 7;
-            const T xw = hw ? xin[i - 1] : (T)0;
-            const T xe = he ? xin[i + 1] : (T)0;
-            const T xm = hm ? xin[i - sb] : (T)0;
-            const T xq = hp ? xin[i + sb] : (T)0;
-            const T xa = u == 0 ? xprev : xc[u > 0 ? u - 1 : 0];           // previous along the line
-            const T xb = u == SEG - 1 ? xnext : xc[u < SEG - 1 ? u + 1 : 0];   // next along the line
-            const bool ha = t > 0, hb = t < L - 1;
-            T acc = a[3] * xc[u];
-            if (DIR == 1) {
-                if (hm) acc += a[0] * xm;                  // z - 1
-                if (ha) acc += a[1] * xa;                  // y - 1
-                if (hw) acc += a[2] * xw;
-                if (he) acc += a[4] * xe;
-                if (hb) acc += a[5] * xb;                  // y + 1
-                if (hp) acc += a[6] * xq;                  // z + 1
-                lv[u] = a[1];
-                uv[u] = a[5] * dv[u];
-            } else {
-                if (ha) acc += a[0] * xa;                  // z - 1
-                if (hm) acc += a[1] * xm;                  // y - 1
-                if (hw) acc += a[2] * xw;
-                if (he) acc += a[4] * xe;
-                if (hp) acc += a[5] * xq;                  // y + 1
-                if (hb) acc += a[6] * xb;                  // z + 1
-                lv[u] = a[0];
-                uv[u] = a[6] * dv[u];
-            }
+    for (int u = 0; u < SEG; u++) same = same && cl[u] == c0;
+    if (ONEROW && __all_sync(lanes, same)) {
+        const T* a = dict + (size_t)c0 * 7;
+        const T a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3], a4 = a[4], a5 = a[5], a6 = a[6];
+#pragma unroll
+        for (int u = 0; u < SEG; u++) {
+            const int i = i0 + (t0 + u) * st;
+            const T xw = xin[i - 1], xe = xin[i + 1], xm = xin[i - sb], xq = xin[i + sb];
+            const T xa = u == 0 ? xprev : xc[u > 0 ? u - 1 : 0];
+            const T xb = u == SEG - 1 ? xnext : xc[u < SEG - 1 ? u + 1 : 0];
+            T acc = a3 * xc[u];
+            acc += a0 * (DIR == 1 ? xm : xa);
+            acc += a1 * (DIR == 1 ? xa : xm);
+            acc += a2 * xw;
+            acc += a4 * xe;
+            acc += a5 * (DIR == 1 ? xb : xq);
+            acc += a6 * (DIR == 1 ? xq : xb);
+            lv[u] = DIR == 1 ? a1 : a0;
+            uv[u] = (DIR == 1 ? a5 : a6) * dv[u];
             rv[u] = rv[u] - acc;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < SEG; u++) {
+            const int t = t0 + u;
+            lv[u] = 0;
+            uv[u] = 0;
+            if (EXACT || t < L) {
+                const int i = i0 + t * st;
+                const T* a = dict + (size_t)cl[u] * 7;
+                const T xw = hw ? xin[i - 1] : (T)0;
+                const T xe = he ? xin[i + 1] : (T)0;
+                const T xm = hm ? xin[i - sb] : (T)0;
+                const T xq = hp ? xin[i + sb] : (T)0;
+                const T xa = u == 0 ? xprev : xc[u > 0 ? u - 1 : 0];           // previous along the line
+                const T xb = u == SEG - 1 ? xnext : xc[u < SEG - 1 ? u + 1 : 0];   // next along the line
+                const bool ha = t > 0, hb = t < L - 1;
+                T acc = a[3] * xc[u];
+                if (DIR == 1) {
+                    if (hm) acc += a[0] * xm;                  // z - 1
+                    if (ha) acc += a[1] * xa;                  // y - 1
+                    if (hw) acc += a[2] * xw;
+                    if (he) acc += a[4] * xe;
+                    if (hb) acc += a[5] * xb;                  // y + 1
+                    if (hp) acc += a[6] * xq;                  // z + 1
+                    lv[u] = a[1];
+                    uv[u] = a[5] * dv[u];
+                } else {
+                    if (ha) acc += a[0] * xa;                  // z - 1
+                    if (hm) acc += a[1] * xm;                  // y - 1
+                    if (hw) acc += a[2] * xw;
+                    if (he) acc += a[4] * xe;
+                    if (hp) acc += a[5] * xq;                  // y + 1
+                    if (hb) acc += a[6] * xb;                  // z + 1
+                    lv[u] = a[0];
+                    uv[u] = a[6] * dv[u];
+                }
+                rv[u] = rv[u] - acc;
+            }
         }
     }
     if (DIR == 2 && zquirk && sg == 0)

@@ -1060,14 +1060,28 @@ static void adlj_fused_step(const LevelT<T>& lv, int d, bool zquirk, T omega, cu
         if (scan) {
             // y-lines that split into whole segments drop the line-end guards
             // (256^3 FP32: 112 against 131 us; the z step measured 140
-            // against 135 us that way and keeps them)
+            // against 135 us that way and keeps them).  On grids of 4M cells
+            // and more FP32 y-lines and FP64 z-lines test for one row per
+            // warp (256^3: 102 against 111 and 214 against 225 us; FP32 z
+            // and FP64 y 145 against 125 and 191 against 164, and at 64^3
+            // FP32 y 6.0 against 4.5).
             const int L = g.M;
             const int sgl = (sizeof(T) == 4 && 8 * ((L + 7) / 8) <= 512) ? 8 : seg_cells<T>(L);
+            const bool big = g.n() >= (1LL << 22);
             if (d == 1) {
-                if (L % sgl == 0) launch_fused_seg<T, 1, 3>(lv, false, omega, s, dinv, xin, xout);
-                else launch_fused_seg<T, 1, 1>(lv, false, omega, s, dinv, xin, xout);
+                if constexpr (sizeof(T) == 4) {
+                    if (big && L % sgl == 0) launch_fused_seg<T, 1, 7>(lv, false, omega, s, dinv, xin, xout);
+                    else if (big) launch_fused_seg<T, 1, 5>(lv, false, omega, s, dinv, xin, xout);
+                }
+                if (sizeof(T) == 8 || !big) {
+                    if (L % sgl == 0) launch_fused_seg<T, 1, 3>(lv, false, omega, s, dinv, xin, xout);
+                    else launch_fused_seg<T, 1, 1>(lv, false, omega, s, dinv, xin, xout);
+                }
             } else {
-                launch_fused_seg<T, 2, 1>(lv, zq, omega, s, dinv, xin, xout);
+                if constexpr (sizeof(T) == 8) {
+                    if (big) launch_fused_seg<T, 2, 5>(lv, zq, omega, s, dinv, xin, xout);
+                }
+                if (sizeof(T) == 4 || !big) launch_fused_seg<T, 2, 1>(lv, zq, omega, s, dinv, xin, xout);
             }
         } else {
             if (d == 1) launch_fused_seg<T, 1, 0>(lv, false, omega, s, dinv, xin, xout);
