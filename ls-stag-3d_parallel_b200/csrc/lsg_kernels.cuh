@@ -505,6 +505,17 @@ __global__ void __launch_bounds__(128) k_applybox8(int N, int M, int K, int rx, 
 // ---------------------------------------------------------------------------
 // transfers (structured tensor-product operators, one 1-D table per axis)
 // ---------------------------------------------------------------------------
+template <typename T>
+struct Vec2;
+template <>
+struct Vec2<float> {
+    using type = float2;
+};
+template <>
+struct Vec2<double> {
+    using type = double2;
+};
+
 // Prolongation table per fine index f: two (coarse index, weight) pairs.
 struct PTab {
     const int* c;      // 2 per fine index
@@ -576,6 +587,119 @@ __global__ void __launch_bounds__(256) k_prolong(int N, int M, int K, int Nc, in
             if (c) c[i] = acc;                             // null: the one copy the fused smoother starts from
         }
     }
+}
+
+// k_prolong where all three fine dimensions are even: a thread owns one coarse
+// column (X, Y), marches over zc coarse planes and writes the 2 x 2 x 2 fine
+// cells of each.  The 3 x 3 coarse values of a plane are loaded once and
+// interpolated along x, y and z in turn (3/4 - 1/4, copied at the ends), so a
+// fine cell costs 9/8 loads and half a vector store instead of eight gathers.
+template <typename T, bool ADD = false>
+__global__ void __launch_bounds__(256) k_prolong_even(int Nc, int Mc, int Kc, int zc, const T* __restrict__ coarse,
+                                                      T* __restrict__ ch, T* __restrict__ c)
+{
+    using V = typename Vec2<T>::type;
+    const int X = blockIdx.x * 32 + threadIdx.x;
+    const int Y = blockIdx.y * 8 + threadIdx.y;
+    if (X >= Nc || Y >= Mc) return;
+    const int z0 = blockIdx.z * zc, z1 = min(z0 + zc, Kc);
+    const int NMc = Nc * Mc, N = 2 * Nc;
+    const long long NMf = 4LL * NMc;                       // cells of a fine plane
+    const bool hw = X > 0, he = X < Nc - 1, hs = Y > 0, hn = Y < Mc - 1;
+    const T q = (T)0.25, t = (T)0.75;
+    int off[9];                                            // rows Y-1, Y, Y+1; a missing neighbour reads the cell
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const int row = (b == 0 ? (hs ? Y - 1 : Y) : (b == 1 ? Y : (hn ? Y + 1 : Y))) * Nc;
+        off[3 * b] = row + (hw ? X - 1 : X);
+        off[3 * b + 1] = row + X;
+        off[3 * b + 2] = row + (he ? X + 1 : X);
+    }
+    auto load = [&](int Z, T* g) {
+        const T* src = coarse + (long long)NMc * min(max(Z, 0), Kc - 1);
+#pragma unroll
+        for (int k = 0; k < 9; k++) g[k] = src[off[k]];
+    };
+    auto plane = [&](const T* g, T* v) {                   // the plane's values at the four fine columns
+        T lo[3], hi[3];
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            lo[b] = hw ? q * g[3 * b] + t * g[3 * b + 1] : g[3 * b + 1];
+            hi[b] = he ? t * g[3 * b + 1] + q * g[3 * b + 2] : g[3 * b + 1];
+        }
+        v[0] = hs ? q * lo[0] + t * lo[1] : lo[1];
+        v[1] = hs ? q * hi[0] + t * hi[1] : hi[1];
+        v[2] = hn ? t * lo[1] + q * lo[2] : lo[1];
+        v[3] = hn ? t * hi[1] + q * hi[2] : hi[1];
+    };
+    T g[9], pm[4], pc[4], pn[4];
+    load(z0 - 1, g);
+    plane(g, pm);
+    load(z0, g);
+    plane(g, pc);
+    load(z0 + 1, g);
+    for (int Z = z0; Z < z1; Z++) {
+        plane(g, pn);
+        if (Z + 1 < z1) load(Z + 2, g);
+        const bool hb = Z > 0, ht = Z < Kc - 1;
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                V v;
+                if (e == 0) {
+                    v.x = hb ? q * pm[2 * r] + t * pc[2 * r] : pc[2 * r];
+                    v.y = hb ? q * pm[2 * r + 1] + t * pc[2 * r + 1] : pc[2 * r + 1];
+                } else {
+                    v.x = ht ? t * pc[2 * r] + q * pn[2 * r] : pc[2 * r];
+                    v.y = ht ? t * pc[2 * r + 1] + q * pn[2 * r + 1] : pc[2 * r + 1];
+                }
+                const long long i = 2 * X + (long long)N * (2 * Y + r) + NMf * (2 * Z + e);
+                V* o = reinterpret_cast<V*>(ch + i);
+                if (ADD) {
+                    const V w = *o;
+                    v.x += w.x;
+                    v.y += w.y;
+                    *o = v;
+                } else {
+                    *o = v;
+                    if (c) *reinterpret_cast<V*>(c + i) = v;
+                }
+            }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            pm[k] = pc[k];
+            pc[k] = pn[k];
+        }
+    }
+}
+
+// The 1/8 agglomeration (all fine dimensions even), x pairs as vectors, summed
+// in k_restrict's order.
+template <typename T>
+__global__ void __launch_bounds__(256) k_restrict_even(int Nc, int Mc, const T* __restrict__ fine,
+                                                       T* __restrict__ coarse)
+{
+    using V = typename Vec2<T>::type;
+    const int X = blockIdx.x * 32 + threadIdx.x;
+    const int Y = blockIdx.y * 8 + threadIdx.y;
+    const int Z = blockIdx.z;
+    if (X >= Nc || Y >= Mc) return;
+    const long long N = 2 * Nc, NM = N * 2 * Mc;
+    const T* f = fine + 2 * X + N * (2 * Y) + NM * (2 * (long long)Z);
+    const V a = *reinterpret_cast<const V*>(f), b = *reinterpret_cast<const V*>(f + N);
+    const V d = *reinterpret_cast<const V*>(f + NM), e = *reinterpret_cast<const V*>(f + NM + N);
+    const T w = (T)0.125;
+    T acc = 0;
+    acc += w * a.x;
+    acc += w * a.y;
+    acc += w * b.x;
+    acc += w * b.y;
+    acc += w * d.x;
+    acc += w * d.y;
+    acc += w * e.x;
+    acc += w * e.y;
+    coarse[X + Nc * (Y + (long long)Mc * Z)] = acc;
 }
 
 // coarse = R fine.  agglomerate: 1/8 of the 2x2x2 block (even-even-even

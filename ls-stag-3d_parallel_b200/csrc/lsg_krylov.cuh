@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(256, 3) k_krylov7z(int N, int M, int K, int zc
 // The same Krylov products with the z planes staged in shared memory (the
 // kernel the solve launches; k_krylov7z stays for timing comparisons): a CTA
 // marches a 32 x 8 (x, y) tile along z with the tile's planes z-1, z, z+1 and
-// their one-cell halo (34 x 10 values) in a ring of three shared buffers, each
+// their one-cell halo (34 x 10 values) in a ring of four shared buffers (one is
+// filled while three are read, so a plane costs one barrier), each
 // plane read once per CTA by two coalesced loads per thread issued one plane
 // ahead; the seven neighbours of a cell then come from shared memory instead
 // of four lateral gathers per cell through L1.  Row class and v stream from
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(256) k_krylov7s(int N, int M, int K, int zc, c
                                                    double* partial, unsigned int* counter, double* out)
 {
     constexpr int TW = 34, TH = 10, TP = TW * TH;
-    __shared__ Tz sp[3][TP];
+    __shared__ Tz sp[4][TP];
     double s[1] = {0.0};
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const int ix = blockIdx.x * 32 + threadIdx.x;
@@ -191,7 +192,7 @@ __global__ void __launch_bounds__(256) k_krylov7s(int N, int M, int K, int zc, c
     int cn = own ? cls[col + NM * z0] : 0;
     double vn = own ? v[col + NM * z0] : 0.0;
     const bool hasw = ix > 0, hase = ix < N - 1, hass = iy > 0, hasn = iy < M - 1;
-    int sm = 0, sc = 1, sn = 2;
+    int sm = 0, sc = 1, sn = 2, sf = 3;
     const int c0 = (threadIdx.y + 1) * TW + threadIdx.x + 1;
     for (int zz = z0; zz < z1; zz++) {
         stage(sn, t);
@@ -223,11 +224,11 @@ __global__ void __launch_bounds__(256) k_krylov7s(int N, int M, int K, int zc, c
                 s[0] += r * r;
             }
         }
-        __syncthreads();
-        const int tt = sm;
+        const int tt = sm;                                 // the plane below is free once the next barrier is passed
         sm = sc;
         sc = sn;
-        sn = tt;
+        sn = sf;
+        sf = tt;
     }
     grid_reduce<1>(s, partial, counter, out);
 }

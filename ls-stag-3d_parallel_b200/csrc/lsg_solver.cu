@@ -1124,6 +1124,40 @@ static void gs_sweep(const LevelT<T>& lv, const T* b, T* x, bool backward, cudaS
     }
 }
 
+// coarse = R fine; the vector form where every fine dimension is even.
+template <typename T>
+static void restrict_level(const Dims& f, const Dims& c, bool even, const TransferTabs& t, const T* fine, T* coarse,
+                           cudaStream_t s)
+{
+    if (even && c.K <= 65535)
+        k_restrict_even<T><<<dim3((c.N + 31) / 32, (c.M + 7) / 8, c.K), dim3(32, 8), 0, s>>>(c.N, c.M, fine, coarse);
+    else
+        k_restrict<T><<<grid_for(c.n(), 256), 256, 0, s>>>(c.N, c.M, c.K, f.N, f.M, even, t.R(0), t.R(1), t.R(2), fine,
+                                                          coarse);
+    LSG_CHECK_LAUNCH();
+}
+
+// ch = P coarse (and c, if given, the same), or ch += P coarse (ADD).  The
+// 2 x 2 x 2 form where every fine dimension is even, 8 coarse planes a thread
+// on levels with work for the whole GPU, fewer on small ones; k_prolong
+// elsewhere.
+template <typename T, bool ADD>
+static void prolong_level(const Dims& f, const Dims& c, bool even, const TransferTabs& t, const T* coarse, T* ch, T* cc,
+                          cudaStream_t s)
+{
+    if (even) {
+        const int zc = c.n() >= (1LL << 20) ? 8 : (c.n() >= (1LL << 17) ? 4 : 1);
+        const dim3 g((c.N + 31) / 32, (c.M + 7) / 8, (c.K + zc - 1) / zc);
+        k_prolong_even<T, ADD><<<g, dim3(32, 8), 0, s>>>(c.N, c.M, c.K, zc, coarse, ch, cc);
+    } else {
+        constexpr int PZ = 4;
+        const dim3 g((f.N + 31) / 32, (f.M + 7) / 8, (f.K + PZ - 1) / PZ);
+        k_prolong<T, PZ, ADD><<<g, dim3(32, 8), 0, s>>>(f.N, f.M, f.K, c.N, c.M, t.P(0), t.P(1), t.P(2), coarse, ch,
+                                                        cc);
+    }
+    LSG_CHECK_LAUNCH();
+}
+
 // V(n_pre, n_post) cycle with the multi-colour Gauss-Seidel smoother (the
 // red-black variant): on the way down each level starts from zero, is
 // pre-smoothed, and restricts its residual; the coarsest level is solved by
@@ -1152,9 +1186,7 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
             res = lv.c.p;
         }
         const TransferTabs& t = mg.tabs[l];
-        k_restrict<T><<<grid_for(c.n(), 256), 256, 0, s>>>(c.N, c.M, c.K, f.N, f.M, mg.agg[l], t.R(0), t.R(1), t.R(2),
-                                                          res, lev[l + 1].r.p);
-        LSG_CHECK_LAUNCH();
+        restrict_level<T>(f, c, mg.agg[l], t, res, lev[l + 1].r.p, s);
     }
     k_coarse_solve<T><<<1, 32, 0, s>>>(mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
                                        mg.dwork.p);
@@ -1164,16 +1196,8 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
         const Dims& f = lv.d;
         const TransferTabs& t = mg.tabs[l];
         T* x = (l == 0 && ch0) ? ch0 : lv.ch.p;
-        constexpr int PZ = 4;
-        const dim3 pg((f.N + 31) / 32, (f.M + 7) / 8, (f.K + PZ - 1) / PZ);
-        if (npre > 0) {
-            k_prolong<T, PZ, true><<<pg, dim3(32, 8), 0, s>>>(f.N, f.M, f.K, lev[l + 1].d.N, lev[l + 1].d.M, t.P(0),
-                                                              t.P(1), t.P(2), lev[l + 1].ch.p, x, lv.c.p);
-        } else {
-            k_prolong<T, PZ><<<pg, dim3(32, 8), 0, s>>>(f.N, f.M, f.K, lev[l + 1].d.N, lev[l + 1].d.M, t.P(0), t.P(1),
-                                                        t.P(2), lev[l + 1].ch.p, x, lv.c.p);
-        }
-        LSG_CHECK_LAUNCH();
+        if (npre > 0) prolong_level<T, true>(f, lev[l + 1].d, mg.agg[l], t, lev[l + 1].ch.p, x, nullptr, s);
+        else prolong_level<T, false>(f, lev[l + 1].d, mg.agg[l], t, lev[l + 1].ch.p, x, lv.c.p, s);
         for (int it = 0; it < npost; it++) gs_sweep<T>(lv, lv.r.p, x, true, s);
     }
     C.vcycles++;
@@ -1208,9 +1232,7 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr, bo
         const Dims& f = lev[l].d;
         const Dims& c = lev[l + 1].d;
         const TransferTabs& t = mg.tabs[l];
-        k_restrict<T><<<grid_for(c.n(), 256), 256, 0, s>>>(c.N, c.M, c.K, f.N, f.M, mg.agg[l], t.R(0), t.R(1), t.R(2),
-                                                          lev[l].r.p, lev[l + 1].r.p);
-        LSG_CHECK_LAUNCH();
+        restrict_level<T>(f, c, mg.agg[l], t, lev[l].r.p, lev[l + 1].r.p, s);
     }
     if (lt >= 0) {
         if constexpr (sizeof(T) == 8) k_vcycle_tail<double><<<1, kTailThreads, 0, s>>>(mg.tail64.p);
@@ -1235,15 +1257,8 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr, bo
         // that one only; the reference schedule needs P c_H in both
         T* buf[2] = {chl, lv.c.p};
         int cur = steps % 2;
-        constexpr int PZ = 4;
-        const dim3 pg((f.N + 31) / 32, (f.M + 7) / 8, (f.K + PZ - 1) / PZ);
-        if (fused)
-            k_prolong<T, PZ><<<pg, dim3(32, 8), 0, s>>>(f.N, f.M, f.K, lev[l + 1].d.N, lev[l + 1].d.M, t.P(0), t.P(1),
-                                                        t.P(2), lev[l + 1].ch.p, buf[cur], nullptr);
-        else
-            k_prolong<T, PZ><<<pg, dim3(32, 8), 0, s>>>(f.N, f.M, f.K, lev[l + 1].d.N, lev[l + 1].d.M, t.P(0), t.P(1),
-                                                        t.P(2), lev[l + 1].ch.p, chl, lv.c.p);
-        LSG_CHECK_LAUNCH();
+        prolong_level<T, false>(f, lev[l + 1].d, mg.agg[l], t, lev[l + 1].ch.p, fused ? buf[cur] : chl,
+                                fused ? nullptr : lv.c.p, s);
         if (fused) {
             for (int it = 0; it < C.opt.n_post; it++)
                 for (int q = 0; q < 3; q++) {
