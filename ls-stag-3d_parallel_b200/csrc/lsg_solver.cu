@@ -174,6 +174,7 @@ struct MGData {
     // lower part of the cycle fused into k_vcycle_tail from level tail_l0 on
     // (-1: every level runs as separate kernels)
     int tail_l0 = -1;
+    size_t tail_smem64 = 0, tail_smem32 = 0;   // its shared memory, bytes
     DevBuf<TailArgs<double>> tail64;
     DevBuf<TailArgs<float>> tail32;
     // the ADLJ V-cycle as one CUDA graph per precision (instantiated on first
@@ -559,9 +560,8 @@ static void fill_tail(const MGData& mg, const std::vector<LevelT<T>>& lev, int l
             t.dinv[d] = lv.dinv[d].p;
             t.up[d] = lv.up[d].p;
         }
-        t.r = const_cast<T*>(lv.r.p);
-        t.c = const_cast<T*>(lv.c.p);
-        t.ch = const_cast<T*>(lv.ch.p);
+        t.r = lv.r.p;
+        t.ch = lv.ch.p;
         if (l < L) {
             const TransferTabs& tb = mg.tabs[l];
             t.px = tb.P(0);
@@ -591,11 +591,19 @@ static void tail_setup(Context& C)
     if (mg.tail_l0 < 0) return;
     TailArgs<double> a64;
     fill_tail<double>(mg, mg.l64, mg.tail_l0, C, a64);
+    mg.tail_smem64 = tail_layout(a64) * sizeof(double);
+    if (mg.tail_smem64 > (size_t)kTailMaxSmem) {        // a level of slivers: separate launches
+        mg.tail_l0 = -1;
+        return;
+    }
+    LSG_CUDA(cudaFuncSetAttribute(k_vcycle_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
+    LSG_CUDA(cudaFuncSetAttribute(k_vcycle_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
     mg.tail64.alloc(1);
     LSG_CUDA(cudaMemcpyAsync(mg.tail64.p, &a64, sizeof(a64), cudaMemcpyHostToDevice, C.s));
     if (mg.fp32) {
         TailArgs<float> a32;
         fill_tail<float>(mg, mg.l32, mg.tail_l0, C, a32);
+        mg.tail_smem32 = tail_layout(a32) * sizeof(float);
         mg.tail32.alloc(1);
         LSG_CUDA(cudaMemcpyAsync(mg.tail32.p, &a32, sizeof(a32), cudaMemcpyHostToDevice, C.s));
     }
@@ -1235,8 +1243,8 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr, bo
         restrict_level<T>(f, c, mg.agg[l], t, lev[l].r.p, lev[l + 1].r.p, s);
     }
     if (lt >= 0) {
-        if constexpr (sizeof(T) == 8) k_vcycle_tail<double><<<1, kTailThreads, 0, s>>>(mg.tail64.p);
-        else k_vcycle_tail<float><<<1, kTailThreads, 0, s>>>(mg.tail32.p);
+        if constexpr (sizeof(T) == 8) k_vcycle_tail<double><<<1, kTailThreads, mg.tail_smem64, s>>>(mg.tail64.p);
+        else k_vcycle_tail<float><<<1, kTailThreads, mg.tail_smem32, s>>>(mg.tail32.p);
     } else {
         k_coarse_solve<T><<<1, 32, 0, s>>>(mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
                                            mg.dwork.p);
