@@ -79,10 +79,10 @@ __device__ __forceinline__ T warp_sum(T v)
 
 // Deterministic block + grid reduction of NS values.  Every block writes its
 // partial sums; the last block to finish adds them in block order and writes
-// out[s].  Blocks of 1-3 dimensions with a multiple of 32 threads (<= 1024),
+// out[s].  Returns true in that block's threads.  Blocks of 1-3 dimensions with a multiple of 32 threads (<= 1024),
 // grids of 1-3 dimensions; blocks and threads are taken in linear order.
 template <int NS>
-__device__ void grid_reduce(double (&v)[NS], double* partial, unsigned int* counter, double* out)
+__device__ bool grid_reduce(double (&v)[NS], double* partial, unsigned int* counter, double* out)
 {
     __shared__ double sh[32][NS];
     __shared__ bool last;
@@ -109,7 +109,7 @@ __device__ void grid_reduce(double (&v)[NS], double* partial, unsigned int* coun
         last = (prev == nblk - 1);
     }
     __syncthreads();
-    if (!last) return;
+    if (!last) return false;
     __threadfence();
     // partials read past L1 (__ldcg), two blocks per step so loads overlap
     double acc[NS];
@@ -143,6 +143,7 @@ __device__ void grid_reduce(double (&v)[NS], double* partial, unsigned int* coun
         }
         *counter = 0u;
     }
+    return true;
 }
 
 // ---------------------------------------------------------------------------

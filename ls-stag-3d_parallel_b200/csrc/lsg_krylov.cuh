@@ -233,13 +233,77 @@ __global__ void __launch_bounds__(256) k_krylov7s(int N, int M, int K, int zc, c
     grid_reduce<1>(s, partial, counter, out);
 }
 
+// What the last kernel of an Arnoldi step needs for the Givens update; ks null:
+// nothing to do.
+struct GivensArgs {
+    KrylovScalars* ks;
+    int j, ldh, max_it;
+    double eps;
+    int* host_flag;        // mapped host memory
+    double* host_norm;
+};
+
+// Givens update of Hessenberg column j and the residual estimate
+// (fgmres_interface.h:103-135), by the first warp of the block that holds the
+// finished ||w||^2.  The lanes read the column and the rotations together (as
+// a one-thread kernel of dependent loads it took 5 us a step); the rotations
+// follow each other in lane 0.
+__device__ __forceinline__ void givens_update(const GivensArgs& g)
+{
+    __shared__ double sH[65], sc[64], ss[64];
+    KrylovScalars* ks = g.ks;
+    const int j = g.j, lane = threadIdx.x;
+    if (lane >= 32) return;
+    volatile double* H = ks->H + (size_t)j * g.ldh;        // its last entry may be this block's own
+    for (int i = lane; i <= j; i += 32) {
+        sH[i] = H[i];
+        sc[i] = i < j ? ks->cs[i] : 0.0;
+        ss[i] = i < j ? ks->sn[i] : 0.0;
+    }
+    __syncwarp();
+    if (lane != 0) return;
+    double curH = sH[0];
+    for (int i = 0; i < j; i++) {
+        const double c = sc[i], s = ss[i];
+        const double nextH = sH[i + 1];
+        H[i] = c * curH - s * nextH;
+        curH = s * curH + c * nextH;
+    }
+    const double normW = sqrt(*(volatile double*)&ks->normW2);
+    const double curC0 = curH * curH + normW * normW;
+    const double curA = sqrt(curC0);
+    double curC = 1.0 / curA;
+    const double curS = -normW * curC;
+    curC *= curH;
+    H[j] = curA;
+    ks->y[j] = curC * ks->norm_r;
+    ks->norm_r *= curS;
+    const double gn = fabs(ks->norm_r);
+    ks->invNormW = 1.0 / normW;
+    int done = 0;
+    if ((gn > g.eps) && (ks->it < g.max_it)) {
+        ks->cs[j] = curC;
+        ks->sn[j] = curS;
+        ks->it++;            // the inner loop's  it++
+    } else {
+        done = 1;
+        ks->norm_r = gn;
+    }
+    if (!(curA > 0.0) || isnan(gn)) ks->breakdown = 1;
+    ks->done = done;
+    *(volatile double*)g.host_norm = gn;
+    __threadfence_system();
+    *(volatile int*)g.host_flag = done ? 2 : 1;
+}
+
 // One modified Gram-Schmidt step fused with the next dot:
-//   w -= h_prev * vprev ;  out = (w, vnext)   (vnext == w gives ||w||^2)
+//   w -= h_prev * vprev ;  out = (w, vnext)   (vnext == w gives ||w||^2);
+// the step that finishes ||w||^2 also does the Givens update (giv).
 __global__ void __launch_bounds__(256) k_mgs_step(long long n, const double* __restrict__ hprev,
                                                    const double* __restrict__ vprev,
                                                    const double* __restrict__ vnext, double* __restrict__ w,
                                                    bool norm_only, double* partial, unsigned int* counter,
-                                                   double* out)
+                                                   double* out, GivensArgs giv)
 {
     const double h = *hprev;
     double s[1] = {0.0};
@@ -249,7 +313,10 @@ __global__ void __launch_bounds__(256) k_mgs_step(long long n, const double* __r
         w[i] = v;
         s[0] += norm_only ? v * v : v * vnext[i];
     }
-    grid_reduce<1>(s, partial, counter, out);
+    if (grid_reduce<1>(s, partial, counter, out) && giv.ks) {
+        __syncthreads();                                   // the norm is written
+        givens_update(giv);
+    }
 }
 
 // v = w / ||w||  (copyTo(curV, normW), mesh_function.h:256-260) and the
@@ -265,47 +332,6 @@ __global__ void k_scale_copy(long long n, const double* __restrict__ w, const do
         v[i] = t;
         if (rhs) rhs[i] = (T)t;
     }
-}
-
-// Givens update of Hessenberg column j and the residual estimate
-// (fgmres_interface.h:103-135).  Runs on one thread.
-__global__ void k_givens(KrylovScalars* ks, int j, int ldh, double eps, int max_it, volatile int* host_flag,
-                         volatile double* host_norm)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double* H = ks->H + (size_t)j * ldh;
-    double curH = H[0];
-    for (int i = 0; i < j; i++) {
-        const double c = ks->cs[i], s = ks->sn[i];
-        const double nextH = H[i + 1];
-        H[i] = c * curH - s * nextH;
-        curH = s * curH + c * nextH;
-    }
-    const double normW = sqrt(ks->normW2);
-    const double curC0 = curH * curH + normW * normW;
-    const double curA = sqrt(curC0);
-    double curC = 1.0 / curA;
-    const double curS = -normW * curC;
-    curC *= curH;
-    H[j] = curA;
-    ks->y[j] = curC * ks->norm_r;
-    ks->norm_r *= curS;
-    const double g = fabs(ks->norm_r);
-    ks->invNormW = 1.0 / normW;
-    int done = 0;
-    if ((g > eps) && (ks->it < max_it)) {
-        ks->cs[j] = curC;
-        ks->sn[j] = curS;
-        ks->it++;            // the inner loop's  it++
-    } else {
-        done = 1;
-        ks->norm_r = g;
-    }
-    if (!(curA > 0.0) || isnan(g)) ks->breakdown = 1;
-    ks->done = done;
-    *host_norm = g;
-    __threadfence_system();
-    *host_flag = done ? 2 : 1;
 }
 
 // Back substitution of the triangular Hessenberg (solUpdate,
@@ -489,34 +515,24 @@ namespace lsg {
 // ---------------------------------------------------------------------------
 constexpr int kGsMaxVec = 64;
 
-// Triangular correction on one thread: store row j of L (from g), solve
-// (I + L) h = s, write h into Hessenberg column j.
-__global__ void k_gs_tri(KrylovScalars* ks, int j, int ldh, const double* __restrict__ sg, double* __restrict__ Lrows)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const double* s = sg;
-    const double* g = sg + (j + 1);
-    for (int k = 0; k < j; k++) Lrows[(size_t)j * kGsMaxVec + k] = g[k];
-    double* H = ks->H + (size_t)j * ldh;
-    for (int i = 0; i <= j; i++) {
-        double h = s[i];
-        for (int k = 0; k < i; k++) h -= Lrows[(size_t)i * kGsMaxVec + k] * H[k];
-        H[i] = h;
-    }
-}
-
 // One pass over V[0..j] and w for the low-synchronisation Gram-Schmidt:
-// s_k = (v_k, w) for k <= j and g_k = (v_k, v_j) for k < j; out = s_0..s_j,
-// g_0..g_{j-1}.  A block is 32 lanes (consecutive cells) by one warp per group
-// of four basis vectors: each warp streams only its own vectors, while w and
-// v_j are shared by the warps of the block through L1.  Per-block sums go to
-// partial[block][q]; the last block to finish adds them in block order.
+// s_k = (v_k, w) for k <= j and g_k = (v_k, v_j) for k < j, then the triangular
+// correction: row j of L is g, and (I + L) h = s gives Hessenberg column j.
+// A block is 32 lanes (consecutive cells) by one warp per group of four basis
+// vectors, by as many cell slices (z) as make about 8 warps: each warp streams
+// only its own vectors, while w and v_j are shared by the warps of a slice
+// through L1.  The slices' sums are added in shared memory, the blocks' by the
+// last block to finish, all in a fixed order.  (Blocks of one slice left that
+// block one warp per four vectors to add up to 4736 partial sums: about 20 us a
+// step at any size.)
 __global__ void __launch_bounds__(512) k_gs_dots2(long long n, long long ld, int j, const double* __restrict__ V,
                                                   const double* __restrict__ w, double* partial,
-                                                  unsigned int* counter, double* out)
+                                                  unsigned int* counter, KrylovScalars* ks, int ldh, double* Lrows)
 {
     constexpr int VW = 4;
-    const int lane = threadIdx.x, grp = threadIdx.y;
+    const int lane = threadIdx.x, grp = threadIdx.y, sl = threadIdx.z;
+    const int groups = blockDim.y, slices = blockDim.z;
+    const int warp = sl * groups + grp, warps = groups * slices;
     const int k0 = grp * VW;
     const int nk = max(0, min(VW, j + 1 - k0));
     double sa[VW], ga[VW];
@@ -526,10 +542,11 @@ __global__ void __launch_bounds__(512) k_gs_dots2(long long n, long long ld, int
         ga[q] = 0.0;
     }
     const double* vj = V + (size_t)j * ld;
-    // each block streams one contiguous range of cells, 128 per warp step
+    // each slice streams one contiguous range of cells, 128 per warp step
     // (four 32-cell pieces, all loads of a step issued before the sums)
-    const long long chunk = ((n + gridDim.x - 1) / gridDim.x + 127) / 128 * 128;
-    const long long beg = (long long)blockIdx.x * chunk, end = min(n, beg + chunk);
+    const long long parts = (long long)gridDim.x * slices;
+    const long long chunk = ((n + parts - 1) / parts + 127) / 128 * 128;
+    const long long beg = ((long long)blockIdx.x * slices + sl) * chunk, end = min(n, beg + chunk);
     for (long long i0 = beg + lane; i0 < end; i0 += 128) {
         double wv[4], vv[4], av[VW][4];
 #pragma unroll
@@ -549,49 +566,72 @@ __global__ void __launch_bounds__(512) k_gs_dots2(long long n, long long ld, int
                 ga[q] += av[q][p] * vv[p];
             }
     }
-    const int pstride = 2 * kGsMaxVec;
+    constexpr int pstride = 2 * kGsMaxVec;
+    __shared__ double sh[16][2 * VW];                      // [warp][sums of its vectors]
+    __shared__ double res[pstride];
+    __shared__ bool last;
 #pragma unroll
     for (int q = 0; q < VW; q++) {
-        sa[q] = warp_sum(sa[q]);
-        ga[q] = warp_sum(ga[q]);
-    }
-    if (lane == 0) {
-        for (int q = 0; q < nk; q++) {
-            const int k = k0 + q;
-            partial[(size_t)blockIdx.x * pstride + k] = sa[q];
-            if (k < j) partial[(size_t)blockIdx.x * pstride + j + 1 + k] = ga[q];
+        const double a = warp_sum(sa[q]), g = warp_sum(ga[q]);
+        if (lane == 0) {
+            sh[warp][q] = a;
+            sh[warp][VW + q] = g;
         }
+    }
+    __syncthreads();
+    const int tid = warp * 32 + lane;
+    if (tid < 2 * VW * groups) {                           // one thread per sum: over the slices, to the partials
+        const int gq = tid / (2 * VW), q = tid - gq * 2 * VW, k = gq * VW + (q & (VW - 1));
+        double t = 0.0;
+        for (int z = 0; z < slices; z++) t += sh[z * groups + gq][q];
+        if (q < VW && k <= j) partial[(size_t)blockIdx.x * pstride + k] = t;
+        if (q >= VW && k < j) partial[(size_t)blockIdx.x * pstride + j + 1 + k] = t;
         __threadfence();
     }
-    __shared__ bool last;
     __syncthreads();
-    if (lane == 0 && grp == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+    if (tid == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // final sums: one warp per value, four independent L2 loads in flight per lane
+    // final sums: one warp per value, eight independent L2 loads in flight per lane
     const int nv = 2 * j + 1;
-    for (int q = grp; q < nv; q += blockDim.y) {
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-        int b = lane;
-        for (; b + 96 < (int)gridDim.x; b += 128) {
-            a0 += __ldcg(partial + (size_t)b * pstride + q);
-            a1 += __ldcg(partial + (size_t)(b + 32) * pstride + q);
-            a2 += __ldcg(partial + (size_t)(b + 64) * pstride + q);
-            a3 += __ldcg(partial + (size_t)(b + 96) * pstride + q);
+    for (int q = warp; q < nv; q += warps) {
+        double a[8] = {};
+        for (int b = lane; b < (int)gridDim.x; b += 256) {
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (b + 32 * u < (int)gridDim.x) a[u] += __ldcg(partial + (size_t)(b + 32 * u) * pstride + q);
         }
-        for (; b < (int)gridDim.x; b += 32) a0 += __ldcg(partial + (size_t)b * pstride + q);
-        const double acc = warp_sum((a0 + a1) + (a2 + a3));
-        if (lane == 0) out[q] = acc;
+        const double acc = warp_sum(((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7])));
+        if (lane == 0) res[q] = acc;
     }
     __syncthreads();
-    if (lane == 0 && grp == 0) *counter = 0u;
+    if (warp != 0) return;
+    if (lane == 0) *counter = 0u;
+    // (I + L) h = s by columns, lane i holding h_i and h_{i+32}
+    const double* g = res + j + 1;
+    double h0 = lane <= j ? res[lane] : 0.0, h1 = lane + 32 <= j ? res[lane + 32] : 0.0;
+    const double* L0 = Lrows + (size_t)lane * kGsMaxVec;
+    const double* L1 = Lrows + (size_t)(lane + 32) * kGsMaxVec;
+    for (int k = 0; k < j; k++) {
+        const double l0 = lane > k && lane <= j ? (lane == j ? g[k] : L0[k]) : 0.0;
+        const double l1 = lane + 32 > k && lane + 32 <= j ? (lane + 32 == j ? g[k] : L1[k]) : 0.0;
+        const double hk = __shfl_sync(0xffffffffu, k < 32 ? h0 : h1, k & 31);
+        h0 -= l0 * hk;
+        h1 -= l1 * hk;
+    }
+    double* H = ks->H + (size_t)j * ldh;
+    if (lane <= j) H[lane] = h0;
+    if (lane + 32 <= j) H[lane + 32] = h1;
+    for (int k = lane; k < j; k += 32) Lrows[(size_t)j * kGsMaxVec + k] = g[k];
 }
 
-// w -= sum_{k<=j} h_k v_k and ||w||^2, the basis vectors read four at a time.
+// w -= sum_{k<=j} h_k v_k and ||w||^2, the basis vectors read four at a time,
+// then the Givens update (giv).
 __global__ void __launch_bounds__(256) k_gs_update2(long long n, long long ld, int j, const double* __restrict__ V,
                                                     const double* __restrict__ h, double* __restrict__ w,
-                                                    double* partial, unsigned int* counter, double* out)
+                                                    double* partial, unsigned int* counter, double* out,
+                                                    GivensArgs giv)
 {
     __shared__ double hs[kGsMaxVec];
     for (int t = threadIdx.x; t <= j; t += blockDim.x) hs[t] = h[t];
@@ -614,7 +654,10 @@ __global__ void __launch_bounds__(256) k_gs_update2(long long n, long long ld, i
         w[i] = acc;
         s[0] += acc * acc;
     }
-    grid_reduce<1>(s, partial, counter, out);
+    if (grid_reduce<1>(s, partial, counter, out) && giv.ks) {
+        __syncthreads();                                   // the norm is written
+        givens_update(giv);
+    }
 }
 
 }  // namespace lsg

@@ -226,7 +226,7 @@ struct Context {
     double* hnorm = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     DevBuf<float> Z32;        // FP32 preconditioned basis (FP32 multigrid)
-    DevBuf<double> gs_partial, gs_sg, gs_L;   // low-synchronisation Gram-Schmidt
+    DevBuf<double> gs_partial, gs_L;   // low-synchronisation Gram-Schmidt
     // ILU(0)
     DevBuf<double> iluL, iluU;        // 3 lower planes (b s w; natural-order sweeps only), pivots
     bool have_ilu = false;
@@ -1415,10 +1415,17 @@ static void precond_apply(Context& C, const double* v, double* z)
 // ---------------------------------------------------------------------------
 // FGMRES (FGMRESInterface::solve, fgmres_interface.h:78-142)
 // ---------------------------------------------------------------------------
-static void launch_givens(Context& C, int j)
+static GivensArgs givens_args(const Context& C, int j)
 {
-    k_givens<<<1, 32, 0, C.s>>>(C.ks.p, j, 65, C.opt.eps, C.opt.max_it, C.hflag, C.hnorm);
-    LSG_CHECK_LAUNCH();
+    GivensArgs g;
+    g.ks = C.ks.p;
+    g.j = j;
+    g.ldh = 65;
+    g.max_it = C.opt.max_it;
+    g.eps = C.opt.eps;
+    g.host_flag = C.hflag;
+    g.host_norm = C.hnorm;
+    return g;
 }
 
 // Low-synchronisation MGS for Arnoldi step j: one pass for V^T w and the new
@@ -1455,16 +1462,14 @@ static void krylov7(Context& C, const Tz* z, const double* v, double* w, double*
 static void gs_lowsync(Context& C, int j, int gb, double* Hj)
 {
     const long long n = C.n;
-    // about 32 resident warps per SM whatever the number of vector groups
-    const int groups = (j + 4) / 4;
-    const int gd = (int)std::min<long long>((n + 127) / 128, std::max(148, 148 * 32 / groups));
-    k_gs_dots2<<<gd, dim3(32, (j + 4) / 4), 0, C.s>>>(n, C.ldv, j, C.V.p, C.w.p, C.gs_partial.p, C.red.counter.p,
-                                                      C.gs_sg.p);
-    LSG_CHECK_LAUNCH();
-    k_gs_tri<<<1, 32, 0, C.s>>>(C.ks.p, j, 65, C.gs_sg.p, C.gs_L.p);
+    // blocks of about 8 warps, three per SM (80 registers), whatever the number of vector groups
+    const int groups = (j + 4) / 4, slices = std::max(1, 8 / groups);
+    const int gd = (int)std::min<long long>((n + 128LL * slices - 1) / (128LL * slices), 148 * 3);
+    k_gs_dots2<<<gd, dim3(32, groups, slices), 0, C.s>>>(n, C.ldv, j, C.V.p, C.w.p, C.gs_partial.p, C.red.counter.p,
+                                                         C.ks.p, 65, C.gs_L.p);
     LSG_CHECK_LAUNCH();
     k_gs_update2<<<gb, 256, 0, C.s>>>(n, C.ldv, j, C.V.p, Hj, C.w.p, C.red.partial.p, C.red.counter.p,
-                                      &C.ks.p->normW2);
+                                      &C.ks.p->normW2, givens_args(C, j));
     LSG_CHECK_LAUNCH();
 }
 
@@ -1543,12 +1548,11 @@ static int fgmres(Context& C, double* x, const double* b, lsg_stats* st)
                         const bool last = (i == j + 1);
                         k_mgs_step<<<gb, 256, 0, s>>>(n, Hj + (i - 1), C.V.p + (size_t)(i - 1) * C.ldv,
                                                      last ? C.w.p : C.V.p + (size_t)i * C.ldv, C.w.p, last, part, cnt,
-                                                     last ? &ks->normW2 : Hj + i);
+                                                     last ? &ks->normW2 : Hj + i, last ? givens_args(C, j) : GivensArgs{});
                         LSG_CHECK_LAUNCH();
                         bytes += (last ? 3 : 4) * w8 * n;
                     }
                 }
-                launch_givens(C, j);
                 LSG_CUDA(cudaStreamSynchronize(s));
                 const int flag = *(volatile int*)C.hflag;
                 if (flag == 2) {
@@ -1886,8 +1890,7 @@ static void krylov_alloc(Context& C)
     C.bd.alloc(n);
     C.coefs.alloc(64);
     if (C.opt.gram_schmidt == LSG_GS_LOWSYNC) {
-        C.gs_partial.alloc((size_t)148 * 32 * 2 * kGsMaxVec);
-        C.gs_sg.alloc(2 * kGsMaxVec);
+        C.gs_partial.alloc((size_t)148 * 3 * 2 * kGsMaxVec);
         C.gs_L.alloc((size_t)kGsMaxVec * kGsMaxVec);
     }
 }
