@@ -114,8 +114,14 @@ __global__ void __launch_bounds__(MAXT, MINB)
         const int t = EXACT ? t0 + u : min(t0 + u, L - 1);
         const int i = i0 + t * st;
         cl[u] = cls[i];
-        rv[u] = b[i];
         dv[u] = dinv[i];
+    }
+    dep_begin(b, xin, xout);                               // the operator does not wait for the step before
+#pragma unroll
+    for (int u = 0; u < SEG; u++) {
+        const int t = EXACT ? t0 + u : min(t0 + u, L - 1);
+        const int i = i0 + t * st;
+        rv[u] = b[i];
         xc[u] = xin[i];
     }
     const T xprev = t0 > 0 ? xin[i0 + (t0 - 1) * st] : (T)0;
@@ -293,9 +299,10 @@ __global__ void __launch_bounds__(256) k_adlj_fused_xseg(int N, int M, int K, in
         cl[4 * k + 2] = c4.z;
         cl[4 * k + 3] = c4.w;
     }
+    load_seg<T, SEG>(dinv + base, dv);
+    dep_begin(b, xin, xout);
     load_seg<T, SEG>(b + base, bv);
     load_seg<T, SEG>(xin + base, xc);
-    load_seg<T, SEG>(dinv + base, dv);
     const bool hzm = z > 0, hym = y > 0, hyp = y < M - 1, hzp = z < K - 1;
     // lateral rows (a row outside the grid is read from this one and not used)
     load_seg<T, SEG>(xin + (hzm ? base - NM : base), zm);

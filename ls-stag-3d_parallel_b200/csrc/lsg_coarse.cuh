@@ -305,7 +305,6 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_tail(const TailArgs<
     const int n0 = v0.N * v0.M * v0.K;
     T a[28];
     if (tid < n0) load_row28(v0.dict28 + (size_t)v0.cls[tid] * 28, a);
-    for (int i = tid; i < n0; i += kTailThreads) sm[v0.s_r + i] = v0.r[i];
     for (int l = 0; l <= last; l++) {
         const TailLevel<T>& v = A.lev[l];
         const int n = v.N * v.M * v.K, nb = tail_box(v.N, v.M, v.K);
@@ -329,6 +328,8 @@ __global__ void __launch_bounds__(kTailThreads, 1) k_vcycle_tail(const TailArgs<
             lu[j * (kTailDense + 1) + i] = A.L[e];
             lu[(kTailDense + j) * (kTailDense + 1) + i] = A.U[e];
         }
+    dep_begin();                                    // all of the above is the operator's
+    for (int i = tid; i < n0; i += kTailThreads) sm[v0.s_r + i] = v0.r[i];
     __syncthreads();
     for (int l = 0; l < last; l++) {
         tail_restrict<T>(A.lev[l], A.lev[l + 1], sm);

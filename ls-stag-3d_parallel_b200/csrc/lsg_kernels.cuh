@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(256) k_apply7z(int N, int M, int K, int zc, co
                                                   const T* __restrict__ dict, const T* __restrict__ x,
                                                   T* __restrict__ r)
 {
+    dep_begin(x, r);
     constexpr int U = 4;
     const int ix = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * 8 + threadIdx.y;
@@ -353,6 +354,7 @@ __global__ void __launch_bounds__(256) k_apply27z(int N, int M, int K, int zc, c
                                                    const T* __restrict__ dict28, const T* __restrict__ x,
                                                    T* __restrict__ r)
 {
+    dep_begin(x, r);
     const int ix = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * 8 + threadIdx.y;
     if (ix >= N || iy >= M) return;
@@ -436,6 +438,7 @@ __global__ void __launch_bounds__(128) k_applybox(int N, int M, int K, const int
                                                    const T* __restrict__ dict, const T* __restrict__ x,
                                                    T* __restrict__ r)
 {
+    dep_begin(x, r);
     constexpr int BX = 2 * RX + 1, BY = 2 * RY + 1, BZ = 2 * RZ + 1;
     const int ix = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * 4 + threadIdx.y;
@@ -474,6 +477,7 @@ __global__ void __launch_bounds__(128) k_applybox8(int N, int M, int K, int rx, 
                                                     const int* __restrict__ cls, const T* __restrict__ dict,
                                                     const T* __restrict__ x, T* __restrict__ r)
 {
+    dep_begin(x, r);
     const int bx = 2 * rx + 1, by = 2 * ry + 1, nb = bx * by * (2 * rz + 1);
     const int NM = N * M, n = NM * K;                      // small levels: int
     __shared__ int so[128][4];                             // dx, dy, dz, flat offset (nb <= 125)
@@ -534,6 +538,7 @@ template <typename T, int ZC, bool ADD = false>
 __global__ void __launch_bounds__(256) k_prolong(int N, int M, int K, int Nc, int Mc, PTab px, PTab py, PTab pz,
                                                  const T* __restrict__ coarse, T* __restrict__ ch, T* __restrict__ c)
 {
+    dep_begin(coarse, ch, c);
     // block (32, 8) over (x, y); each thread ZC consecutive z.  All gathers of
     // the ZC cells are issued before any is summed (unused table slots hold
     // index 0 and weight 0, so every address is valid); the sum skips zero
@@ -599,6 +604,7 @@ template <typename T, bool ADD = false>
 __global__ void __launch_bounds__(256) k_prolong_even(int Nc, int Mc, int Kc, int zc, const T* __restrict__ coarse,
                                                       T* __restrict__ ch, T* __restrict__ c)
 {
+    dep_begin(coarse, ch, c);
     using V = typename Vec2<T>::type;
     const int X = blockIdx.x * 32 + threadIdx.x;
     const int Y = blockIdx.y * 8 + threadIdx.y;
@@ -681,6 +687,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_restrict_even(int Nc, int Mc, const T* __restrict__ fine,
                                                        T* __restrict__ coarse)
 {
+    dep_begin(fine, coarse);
     using V = typename Vec2<T>::type;
     const int X = blockIdx.x * 32 + threadIdx.x;
     const int Y = blockIdx.y * 8 + threadIdx.y;
@@ -709,6 +716,7 @@ template <typename T>
 __global__ void k_restrict(int Nc, int Mc, int Kc, int N, int M, bool agglomerate, RTab rx, RTab ry, RTab rz,
                            const T* __restrict__ fine, T* __restrict__ coarse)
 {
+    dep_begin(fine, coarse);
     const long long nc = (long long)Nc * Mc * Kc;
     const int NMc = Nc * Mc, NM = N * M;
     const CellIndex ci(Nc, NMc);
@@ -1001,6 +1009,7 @@ __global__ void __launch_bounds__(128) k_tdma_strided(LineGeom g, bool zquirk, c
                                                        const T* __restrict__ r, T* __restrict__ c,
                                                        T* __restrict__ ch, T omega)
 {
+    dep_begin(r, c, ch);
     constexpr int U = 8;
     const long long nl = g.nlines();
     const int L = g.len();
@@ -1201,10 +1210,16 @@ __global__ void __launch_bounds__(MAXT, MINB) k_tdma_seg(LineGeom g, bool zquirk
     for (int u = 0; u < SEG; u++) {
         const int t = min(t0 + u, L - 1);
         const long long i = i0 + (long long)t * st;
-        rv[u] = r[i];
         lv[u] = lo[i];
         dv[u] = dinv[i];
         uv[u] = up[i];
+    }
+    dep_begin(r, c, ch);                                   // the factors do not wait for the step before
+#pragma unroll
+    for (int u = 0; u < SEG; u++) {
+        const int t = min(t0 + u, L - 1);
+        const long long i = i0 + (long long)t * st;
+        rv[u] = r[i];
         hv[u] = ch[i];
     }
     if (zquirk && sg == 0) rv[0] = r[(long long)row * g.N * g.K + xs];   // reference z-line quirk (y*N*K + x)
@@ -1335,10 +1350,11 @@ __global__ void __launch_bounds__(256) k_tdma_xseg(int L, int P, long long nline
     const bool valid = line < nlines;
     const long long base = (valid ? line : 0) * L + (long long)q * SEG;
     T rv[SEG], lv[SEG], dv[SEG], uv[SEG], hv[SEG];
-    load_seg<T, SEG>(r + base, rv);
     load_seg<T, SEG>(lo + base, lv);
     load_seg<T, SEG>(dinv + base, dv);
     load_seg<T, SEG>(up + base, uv);
+    dep_begin(r, c, ch);
+    load_seg<T, SEG>(r + base, rv);
     load_seg<T, SEG>(ch + base, hv);
     // forward: y_t = (r_t - lo_t y_{t-1}) dinv_t relative to the segment input
     T a = 0, b = 1;
@@ -1415,6 +1431,7 @@ __global__ void __launch_bounds__(256) k_tdma_xwarp(int N, long long nlines, con
                                                      const T* __restrict__ r, T* __restrict__ c,
                                                      T* __restrict__ ch, T omega)
 {
+    dep_begin(r, c, ch);
     const int lane = threadIdx.x & 31;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1509,6 +1526,7 @@ __global__ void k_coarse_solve(int n, const double* __restrict__ L, const double
                                const double* __restrict__ scale, const int* __restrict__ perm,
                                const T* __restrict__ b, T* __restrict__ ch, double* __restrict__ work)
 {
+    dep_begin(b, ch);
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     double* y = work;
     double* z = work + n;
@@ -1661,6 +1679,7 @@ __global__ void __launch_bounds__(256) k_gs_rb7(int N, int M, int K, int color, 
                                                 const T* __restrict__ dict, const T* __restrict__ dinv,
                                                 const T* __restrict__ b, T* __restrict__ x)
 {
+    dep_begin(b, x);
     const int xh = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * 8 + threadIdx.y;
     const int iz = blockIdx.z;
@@ -1686,6 +1705,7 @@ __global__ void __launch_bounds__(256) k_gs_box27(int N, int M, int K, int color
                                                   const T* __restrict__ dict28, const T* __restrict__ dinv,
                                                   const T* __restrict__ b, T* __restrict__ x)
 {
+    dep_begin(b, x);
     const int ix = 2 * (blockIdx.x * 32 + threadIdx.x) + (color & 1);
     const int iy = 2 * (blockIdx.y * 8 + threadIdx.y) + ((color >> 1) & 1);
     const int iz = 2 * blockIdx.z + ((color >> 2) & 1);

@@ -840,12 +840,12 @@ static void apply_box(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s)
                     lv.ol.n == (2 * rx + 1) * (2 * ry + 1) * (2 * rz + 1),
                 LSG_ERR_STATE, "unexpected coarse stencil");
     if (n < 32768) {
-        k_applybox8<T, MODE><<<(unsigned)((n + 15) / 16), 128, 0, s>>>(d.N, d.M, d.K, rx, ry, rz, lv.cls, lv.dict, x,
+        launch_dep(k_applybox8<T, MODE>, (unsigned)((n + 15) / 16), 128, 0, s, d.N, d.M, d.K, rx, ry, rz, lv.cls, lv.dict, x,
                                                                       r);
         return;
     }
     const dim3 b(32, 4), g((d.N + 31) / 32, (d.M + 3) / 4, std::min(d.K, 65535));
-    auto go = [&](auto kernel) { kernel<<<g, b, 0, s>>>(d.N, d.M, d.K, lv.cls, lv.dict, x, r); };
+    auto go = [&](auto kernel) { launch_dep(kernel, g, b, 0, s, d.N, d.M, d.K, lv.cls, lv.dict, x, r); };
     switch (rx * 4 + ry * 2 + rz - 7) {
     case 0: go(k_applybox<T, MODE, 1, 1, 1>); break;
     case 1: go(k_applybox<T, MODE, 1, 1, 2>); break;
@@ -869,14 +869,14 @@ static void apply_resid(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s, i
     const dim3 zb(32, 8), zg((lv.d.N + 31) / 32, (lv.d.M + 7) / 8, (lv.d.K + zc - 1) / zc);
     if (lv.ol.n == 7 && lv.off[0] == 0 && lv.off[2] == -1) {
         if (mode == 0)
-            k_apply7z<T, 0><<<zg, zb, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
+            launch_dep(k_apply7z<T, 0>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
         else
-            k_apply7z<T, 1><<<zg, zb, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
+            launch_dep(k_apply7z<T, 1>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
     } else if (lv.ol.n == 27 && lv.dict28.p) {
         if (mode == 0)
-            k_apply27z<T, 0><<<zg, zb, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
+            launch_dep(k_apply27z<T, 0>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
         else
-            k_apply27z<T, 1><<<zg, zb, 0, s>>>(lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
+            launch_dep(k_apply27z<T, 1>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
     } else if (mode == 0) {
         apply_box<T, 0>(lv, x, r, s);
     } else {
@@ -905,15 +905,15 @@ static void line_solve(const LevelT<T>& lv, int d, bool zquirk, T omega, cudaStr
         const int P8 = xseg_p(8), P12 = xseg_p(12);
         if (aligned && P8) {
             const long long threads = nl * P8;
-            k_tdma_xseg<T, 8><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+            launch_dep(k_tdma_xseg<T, 8>, (unsigned)((threads + 255) / 256), 256, 0, s, 
                 g.N, P8, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p, ch, omega);
         } else if (aligned && P12) {
             const long long threads = nl * P12;
-            k_tdma_xseg<T, 12><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+            launch_dep(k_tdma_xseg<T, 12>, (unsigned)((threads + 255) / 256), 256, 0, s, 
                 g.N, P12, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p, ch, omega);
         } else {
             const int blocks = grid_for(nl * 32, 256, 148 * 64);
-            k_tdma_xwarp<T><<<blocks, 256, 0, s>>>(g.N, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p,
+            launch_dep(k_tdma_xwarp<T>, blocks, 256, 0, s, g.N, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p,
                                                    ch, omega);
         }
     } else {
@@ -938,24 +938,24 @@ static void line_solve(const LevelT<T>& lv, int d, bool zquirk, T omega, cudaStr
         const bool seg4 = (form == 2 || (form == 0 && sizeof(T) == 8 && d == 2)) && 8 * S4 <= 512;
         if (seg4) {
             const long long blocks = (long long)((g.N + 7) / 8) * rows;
-            k_tdma_seg<T, 4, 512, 2><<<(unsigned)blocks, dim3(8, S4), 4 * (size_t)8 * S4 * sizeof(T), s>>>(
+            launch_dep(k_tdma_seg<T, 4, 512, 2>, (unsigned)blocks, dim3(8, S4), 4 * (size_t)8 * S4 * sizeof(T), s, 
                 lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
         } else if (8 * S8 <= MAXT && (S8 <= 32 || 8 * S12 > MAXT)) {
             const int W = pick_w(S8);
             const long long blocks = (long long)((g.N + W - 1) / W) * rows;
             if (walk)
-                k_tdma_seg<T, 8, MAXT, 2, false><<<(unsigned)blocks, dim3(W, S8), 4 * (size_t)W * S8 * sizeof(T), s>>>(
+                launch_dep(k_tdma_seg<T, 8, MAXT, 2, false>, (unsigned)blocks, dim3(W, S8), 4 * (size_t)W * S8 * sizeof(T), s, 
                     lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
             else
-                k_tdma_seg<T, 8, MAXT, 2><<<(unsigned)blocks, dim3(W, S8), 4 * (size_t)W * S8 * sizeof(T), s>>>(
+                launch_dep(k_tdma_seg<T, 8, MAXT, 2>, (unsigned)blocks, dim3(W, S8), 4 * (size_t)W * S8 * sizeof(T), s, 
                     lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
         } else if (sizeof(T) == 4 && 8 * S12 <= MAXT) {
             const int W = pick_w(S12);
             const long long blocks = (long long)((g.N + W - 1) / W) * rows;
-            k_tdma_seg<T, 12, MAXT, 1><<<(unsigned)blocks, dim3(W, S12), 4 * (size_t)W * S12 * sizeof(T), s>>>(
+            launch_dep(k_tdma_seg<T, 12, MAXT, 1>, (unsigned)blocks, dim3(W, S12), 4 * (size_t)W * S12 * sizeof(T), s, 
                 lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
         } else {
-            k_tdma_strided<T><<<grid_for(lg.nlines(), 128, 148 * 64), 128, 0, s>>>(
+            launch_dep(k_tdma_strided<T>, grid_for(lg.nlines(), 128, 148 * 64), 128, 0, s, 
                 lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
         }
     }
@@ -1026,11 +1026,11 @@ static void launch_fused_seg(const LevelT<T>& lv, bool zq, T omega, cudaStream_t
     const size_t sm = 4 * (size_t)W * S * sizeof(T);       // scan buffers
     const T* dict = lv.dict;
     if (seg == 8) {
-        k_adlj_fused_seg<T, DIR, 8, MAXT, 2, VAR><<<blocks, blk, sm, s>>>(g.N, g.M, g.K, zq, lv.cls, dict, dinv,
+        launch_dep(k_adlj_fused_seg<T, DIR, 8, MAXT, 2, VAR>, blocks, blk, sm, s, g.N, g.M, g.K, zq, lv.cls, dict, dinv,
                                                                          lv.r.p, xin, xout, omega);
     } else {
         if constexpr (sizeof(T) == 4)
-            k_adlj_fused_seg<T, DIR, 12, MAXT, 1, VAR><<<blocks, blk, sm, s>>>(g.N, g.M, g.K, zq, lv.cls, dict,
+            launch_dep(k_adlj_fused_seg<T, DIR, 12, MAXT, 1, VAR>, blocks, blk, sm, s, g.N, g.M, g.K, zq, lv.cls, dict,
                                                                               dinv, lv.r.p, xin, xout, omega);
         else
             throw Error{LSG_ERR_STATE, "no fused line kernel for this line length"};
@@ -1053,14 +1053,14 @@ static void adlj_fused_step(const LevelT<T>& lv, int d, bool zquirk, T omega, cu
         const int P = g.N / seg;
         const long long threads = (long long)g.M * g.K * P;
         if (seg == 8)
-            k_adlj_fused_xseg<T, 8><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(g.N, g.M, g.K, P, lv.cls,
+            launch_dep(k_adlj_fused_xseg<T, 8>, (unsigned)((threads + 255) / 256), 256, 0, s, g.N, g.M, g.K, P, lv.cls,
                                                                                     lv.dict, dinv, b, xin, xout, omega);
         else if (seg == 12)
-            k_adlj_fused_xseg<T, 12><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(g.N, g.M, g.K, P, lv.cls,
+            launch_dep(k_adlj_fused_xseg<T, 12>, (unsigned)((threads + 255) / 256), 256, 0, s, g.N, g.M, g.K, P, lv.cls,
                                                                                      lv.dict, dinv, b, xin, xout,
                                                                                      omega);
         else
-            k_adlj_fused_xseg<T, 16><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(g.N, g.M, g.K, P, lv.cls,
+            launch_dep(k_adlj_fused_xseg<T, 16>, (unsigned)((threads + 255) / 256), 256, 0, s, g.N, g.M, g.K, P, lv.cls,
                                                                                      lv.dict, dinv, b, xin, xout,
                                                                                      omega);
     } else {
@@ -1109,14 +1109,14 @@ static void gs_sweep(const LevelT<T>& lv, const T* b, T* x, bool backward, cudaS
     if (lv.ol.n == 7 && lv.off[0] == 0 && lv.off[2] == -1) {
         const dim3 g((d.N / 2 + 1 + 31) / 32, (d.M + 7) / 8, d.K);
         for (int q = 0; q < 2; q++) {
-            k_gs_rb7<T><<<g, dim3(32, 8), 0, s>>>(d.N, d.M, d.K, backward ? 1 - q : q, lv.cls, lv.dict,
+            launch_dep(k_gs_rb7<T>, g, dim3(32, 8), 0, s, d.N, d.M, d.K, backward ? 1 - q : q, lv.cls, lv.dict,
                                                   lv.gsdinv.p, b, x);
             LSG_CHECK_LAUNCH();
         }
     } else if (lv.ol.n == 27 && lv.dict28.p) {
         const dim3 g(((d.N + 1) / 2 + 31) / 32, ((d.M + 1) / 2 + 7) / 8, (d.K + 1) / 2);
         for (int q = 0; q < 8; q++) {
-            k_gs_box27<T><<<g, dim3(32, 8), 0, s>>>(d.N, d.M, d.K, backward ? 7 - q : q, lv.cls, lv.dict28.p,
+            launch_dep(k_gs_box27<T>, g, dim3(32, 8), 0, s, d.N, d.M, d.K, backward ? 7 - q : q, lv.cls, lv.dict28.p,
                                                     lv.gsdinv.p, b, x);
             LSG_CHECK_LAUNCH();
         }
@@ -1138,9 +1138,9 @@ static void restrict_level(const Dims& f, const Dims& c, bool even, const Transf
                            cudaStream_t s)
 {
     if (even && c.K <= 65535)
-        k_restrict_even<T><<<dim3((c.N + 31) / 32, (c.M + 7) / 8, c.K), dim3(32, 8), 0, s>>>(c.N, c.M, fine, coarse);
+        launch_dep(k_restrict_even<T>, dim3((c.N + 31) / 32, (c.M + 7) / 8, c.K), dim3(32, 8), 0, s, c.N, c.M, fine, coarse);
     else
-        k_restrict<T><<<grid_for(c.n(), 256), 256, 0, s>>>(c.N, c.M, c.K, f.N, f.M, even, t.R(0), t.R(1), t.R(2), fine,
+        launch_dep(k_restrict<T>, grid_for(c.n(), 256), 256, 0, s, c.N, c.M, c.K, f.N, f.M, even, t.R(0), t.R(1), t.R(2), fine,
                                                           coarse);
     LSG_CHECK_LAUNCH();
 }
@@ -1156,11 +1156,11 @@ static void prolong_level(const Dims& f, const Dims& c, bool even, const Transfe
     if (even) {
         const int zc = c.n() >= (1LL << 20) ? 8 : (c.n() >= (1LL << 17) ? 4 : 1);
         const dim3 g((c.N + 31) / 32, (c.M + 7) / 8, (c.K + zc - 1) / zc);
-        k_prolong_even<T, ADD><<<g, dim3(32, 8), 0, s>>>(c.N, c.M, c.K, zc, coarse, ch, cc);
+        launch_dep(k_prolong_even<T, ADD>, g, dim3(32, 8), 0, s, c.N, c.M, c.K, zc, coarse, ch, cc);
     } else {
         constexpr int PZ = 4;
         const dim3 g((f.N + 31) / 32, (f.M + 7) / 8, (f.K + PZ - 1) / PZ);
-        k_prolong<T, PZ, ADD><<<g, dim3(32, 8), 0, s>>>(f.N, f.M, f.K, c.N, c.M, t.P(0), t.P(1), t.P(2), coarse, ch,
+        launch_dep(k_prolong<T, PZ, ADD>, g, dim3(32, 8), 0, s, f.N, f.M, f.K, c.N, c.M, t.P(0), t.P(1), t.P(2), coarse, ch,
                                                         cc);
     }
     LSG_CHECK_LAUNCH();
@@ -1196,7 +1196,7 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
         const TransferTabs& t = mg.tabs[l];
         restrict_level<T>(f, c, mg.agg[l], t, res, lev[l + 1].r.p, s);
     }
-    k_coarse_solve<T><<<1, 32, 0, s>>>(mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
+    launch_dep(k_coarse_solve<T>, 1, 32, 0, s, mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
                                        mg.dwork.p);
     LSG_CHECK_LAUNCH();
     for (int l = L - 1; l >= 0; l--) {
@@ -1243,10 +1243,10 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr, bo
         restrict_level<T>(f, c, mg.agg[l], t, lev[l].r.p, lev[l + 1].r.p, s);
     }
     if (lt >= 0) {
-        if constexpr (sizeof(T) == 8) k_vcycle_tail<double><<<1, kTailThreads, mg.tail_smem64, s>>>(mg.tail64.p);
-        else k_vcycle_tail<float><<<1, kTailThreads, mg.tail_smem32, s>>>(mg.tail32.p);
+        if constexpr (sizeof(T) == 8) launch_dep(k_vcycle_tail<double>, 1, kTailThreads, mg.tail_smem64, s, mg.tail64.p);
+        else launch_dep(k_vcycle_tail<float>, 1, kTailThreads, mg.tail_smem32, s, mg.tail32.p);
     } else {
-        k_coarse_solve<T><<<1, 32, 0, s>>>(mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
+        launch_dep(k_coarse_solve<T>, 1, 32, 0, s, mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
                                            mg.dwork.p);
     }
     LSG_CHECK_LAUNCH();
