@@ -988,10 +988,15 @@ static int xseg_cells(int N)
     return 0;
 }
 
+// Segment length of the same step on lines of any other length, 0 = longer
+// than 512.
+static int xany_cells(int N) { return N <= 256 ? 8 : (N <= 384 ? 12 : (N <= 512 ? 16 : 0)); }
+
 // Whether a level with these dimensions and stencil runs the fused ADLJ
 // direction steps: the fine 7-point stencil (offsets b, s, w, p, e, n, t),
-// x-lines of 8-, 12- or 16-cell segments on P <= 32 lanes (P a power of two),
-// y- and z-lines in the segmented kernel's shapes.  Both precisions: a fused
+// x-lines of at most 512 cells (vectors where they are 8-, 12- or 16-cell
+// segments on P <= 32 lanes, P a power of two; scalars otherwise), y- and
+// z-lines in the segmented kernel's shapes.  Both precisions: a fused
 // step moves 4w + 4 bytes a cell where the residual and the line solve move
 // 10w + 4 (256^3 FP64 solve 44.5 against 54.8 ms, the 128 x 64 x 64 time step
 // 4.13 against 4.55 ms).
@@ -1001,7 +1006,7 @@ static bool adlj_fused_level(const Dims& g, int noff, const std::vector<int>& of
     if (o.smoother != LSG_SMOOTHER_ADLJ) return false;
     if (o.adlj_schedule == LSG_ADLJ_REFERENCE) return false;
     if (noff != 7 || off.size() < 3 || off[0] != 0 || off[1] != 0 || off[2] != -1) return false;
-    if (g.N < 2 || g.M < 2 || g.K < 2 || !xseg_cells(g.N)) return false;
+    if (g.N < 2 || g.M < 2 || g.K < 2 || !(xseg_cells(g.N) || xany_cells(g.N))) return false;
     return seg_cells<T>(g.M) != 0 && seg_cells<T>(g.K) != 0;
 }
 
@@ -1049,20 +1054,19 @@ static void adlj_fused_step(const LevelT<T>& lv, int d, bool zquirk, T omega, cu
     const T* b = lv.r.p;
     const T* dinv = lv.dinv[d].p;
     if (d == 0) {
-        const int seg = xseg_cells(g.N);
-        const int P = g.N / seg;
-        const long long threads = (long long)g.M * g.K * P;
-        if (seg == 8)
-            launch_dep(k_adlj_fused_xseg<T, 8>, (unsigned)((threads + 255) / 256), 256, 0, s, g.N, g.M, g.K, P, lv.cls,
-                                                                                    lv.dict, dinv, b, xin, xout, omega);
-        else if (seg == 12)
-            launch_dep(k_adlj_fused_xseg<T, 12>, (unsigned)((threads + 255) / 256), 256, 0, s, g.N, g.M, g.K, P, lv.cls,
-                                                                                     lv.dict, dinv, b, xin, xout,
-                                                                                     omega);
-        else
-            launch_dep(k_adlj_fused_xseg<T, 16>, (unsigned)((threads + 255) / 256), 256, 0, s, g.N, g.M, g.K, P, lv.cls,
-                                                                                     lv.dict, dinv, b, xin, xout,
-                                                                                     omega);
+        const int vec = xseg_cells(g.N), seg = vec ? vec : xany_cells(g.N);
+        int P = 1;
+        while (P * seg < g.N) P *= 2;
+        const unsigned blocks = (unsigned)(((long long)g.M * g.K * P + 255) / 256);
+        auto go = [&](auto kernel) {
+            launch_dep(kernel, blocks, 256, 0, s, g.N, g.M, g.K, P, lv.cls, lv.dict, dinv, b, xin, xout, omega);
+        };
+        if (vec == 8) go(k_adlj_fused_xseg<T, 8>);
+        else if (vec == 12) go(k_adlj_fused_xseg<T, 12>);
+        else if (vec == 16) go(k_adlj_fused_xseg<T, 16>);
+        else if (seg == 8) go(k_adlj_fused_xseg<T, 8, true>);
+        else if (seg == 12) go(k_adlj_fused_xseg<T, 12, true>);
+        else go(k_adlj_fused_xseg<T, 16, true>);
     } else {
         const bool zq = d == 2 && zquirk;
         if (scan) {

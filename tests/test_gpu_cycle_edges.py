@@ -34,7 +34,7 @@ def _case(dims, seed, scale=(1.0, 1.0, 1.0)):
 
 
 DIMS = [(66, 65, 64), (52, 51, 50), (33, 17, 9), (17, 19, 21), (64, 48, 32), (16, 16, 16), (130, 6, 8), (6, 130, 10),
-        (24, 20, 12), (128, 32, 16), (5, 4, 7), (96, 80, 64)]
+        (24, 20, 12), (128, 32, 16), (5, 4, 7), (96, 80, 64), (300, 6, 5), (430, 5, 6), (600, 5, 4)]
 
 
 @pytest.mark.parametrize("dims", DIMS)
