@@ -199,14 +199,26 @@ struct Reducer {
 struct KrylovScalars {
     double H[64 * 65];      // column-major Hessenberg entries h[i + j*65]
     double cs[64], sn[64], y[64];
-    double norm_r;          // running |gamma|
     double normW2;          // ||w||^2 of the latest Arnoldi vector
     double invNormW;        // 1 / ||w||
-    double bnorm2;
-    int it;
+    // what the host reads when a cycle ends
+    struct State {
+        double norm_r;      // running |gamma|
+        int it;
+        int breakdown;
+    } st;
     int done;               // 1 converged / capped
-    int breakdown;
     int pad;
+};
+
+// The host's side of a solve in pinned memory: the flags that the kernels
+// write each step, and the targets of the copies at a solve's end.
+struct HostScalars {
+    int flag;               // mapped: 2 finished, 1 not
+    int ilu_err;
+    double norm;            // mapped: the step's residual estimate
+    double r2;              // ||b - A x||^2
+    KrylovScalars::State st;
 };
 
 // ---------------------------------------------------------------------------

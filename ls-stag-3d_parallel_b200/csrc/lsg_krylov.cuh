@@ -276,20 +276,20 @@ __device__ __forceinline__ void givens_update(const GivensArgs& g)
     const double curS = -normW * curC;
     curC *= curH;
     H[j] = curA;
-    ks->y[j] = curC * ks->norm_r;
-    ks->norm_r *= curS;
-    const double gn = fabs(ks->norm_r);
+    ks->y[j] = curC * ks->st.norm_r;
+    ks->st.norm_r *= curS;
+    const double gn = fabs(ks->st.norm_r);
     ks->invNormW = 1.0 / normW;
     int done = 0;
-    if ((gn > g.eps) && (ks->it < g.max_it)) {
+    if ((gn > g.eps) && (ks->st.it < g.max_it)) {
         ks->cs[j] = curC;
         ks->sn[j] = curS;
-        ks->it++;            // the inner loop's  it++
+        ks->st.it++;            // the inner loop's  it++
     } else {
         done = 1;
-        ks->norm_r = gn;
+        ks->st.norm_r = gn;
     }
-    if (!(curA > 0.0) || isnan(gn)) ks->breakdown = 1;
+    if (!(curA > 0.0) || isnan(gn)) ks->st.breakdown = 1;
     ks->done = done;
     *(volatile double*)g.host_norm = gn;
     __threadfence_system();
@@ -332,6 +332,17 @@ __global__ void k_scale_copy(long long n, const double* __restrict__ w, const do
         v[i] = t;
         if (rhs) rhs[i] = (T)t;
     }
+}
+
+// Start of a cycle from a residual of this norm, in iteration `it`; the first vector is w / norm.
+__global__ void k_krylov_start(KrylovScalars* ks, double norm, int it, bool fresh)
+{
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    ks->st.norm_r = norm;
+    ks->invNormW = 1.0 / norm;
+    ks->done = 0;
+    ks->st.it = it;
+    if (fresh) ks->st.breakdown = 0;
 }
 
 // Back substitution of the triangular Hessenberg (solUpdate,

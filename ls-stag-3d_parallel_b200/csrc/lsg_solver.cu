@@ -222,8 +222,7 @@ struct Context {
     long long ldv = 0;        // stride between basis vectors (n padded off a power of two)
     DevBuf<double> V, Z, w, xd, bd, coefs, t1, t2, t3, t4;
     DevBuf<KrylovScalars> ks;
-    int* hflag = nullptr;
-    double* hnorm = nullptr;
+    HostScalars* host = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     DevBuf<float> Z32;        // FP32 preconditioned basis (FP32 multigrid)
     DevBuf<double> gs_partial, gs_L;   // low-synchronisation Gram-Schmidt
@@ -292,6 +291,8 @@ namespace lsg {
 
 static void ilu_apply(Context& C, const double* b, double* x);
 static void ilu_check(Context& C);
+static void ilu_fetch(Context& C);
+static void ilu_raise(Context& C);
 
 // ---------------------------------------------------------------------------
 // row dictionary of an operator given as noff coefficient planes
@@ -1427,8 +1428,8 @@ static GivensArgs givens_args(const Context& C, int j)
     g.ldh = 65;
     g.max_it = C.opt.max_it;
     g.eps = C.opt.eps;
-    g.host_flag = C.hflag;
-    g.host_norm = C.hnorm;
+    g.host_flag = &C.host->flag;
+    g.host_norm = &C.host->norm;
     return g;
 }
 
@@ -1491,24 +1492,20 @@ static int fgmres(Context& C, double* x, const double* b, lsg_stats* st)
     // norm_r = ||b - A x||  ; w = b - A x
     krylov7<double, 1>(C, x, b, C.w.p, &ks->normW2);
     bytes += (3 * w8 + 4) * n;
-    double nrm2 = 0;
-    LSG_CUDA(cudaMemcpyAsync(&nrm2, &ks->normW2, sizeof(double), cudaMemcpyDeviceToHost, s));
+    LSG_CUDA(cudaMemcpyAsync(&C.host->r2, &ks->normW2, sizeof(double), cudaMemcpyDeviceToHost, s));
     LSG_CUDA(cudaStreamSynchronize(s));
-    double norm_r = std::sqrt(nrm2);
+    double norm_r = std::sqrt(C.host->r2);
     int it = 0;
+    bool breakdown = false;
+    bool have_r2 = false;                   // host->r2 is the FP64 residual of the final x
     int status = LSG_OK;
     // a NaN or Inf in b, x or the operator: no iteration can help (the
     // reference would iterate to MAX_ITER on NaNs and report nothing)
     if (!std::isfinite(norm_r)) status = LSG_BREAKDOWN;
     else if (norm_r > C.opt.eps) {
         it = 1;
-        // initialise device scalars: norm_r, invNormW = 1/norm_r, it
-        KrylovScalars h;
-        std::memset(&h, 0, sizeof(h));
-        h.norm_r = norm_r;
-        h.invNormW = 1.0 / norm_r;
-        h.it = 1;
-        LSG_CUDA(cudaMemcpyAsync(ks, &h, sizeof(h), cudaMemcpyHostToDevice, s));
+        k_krylov_start<<<1, 32, 0, s>>>(ks, norm_r, 1, true);
+        LSG_CHECK_LAUNCH();
         bool finished = false;
         while (!finished) {
             int jlast = m - 1;
@@ -1558,7 +1555,7 @@ static int fgmres(Context& C, double* x, const double* b, lsg_stats* st)
                     }
                 }
                 LSG_CUDA(cudaStreamSynchronize(s));
-                const int flag = *(volatile int*)C.hflag;
+                const int flag = *(volatile int*)&C.host->flag;
                 if (flag == 2) {
                     jlast = j;
                     finished = true;
@@ -1580,44 +1577,58 @@ static int fgmres(Context& C, double* x, const double* b, lsg_stats* st)
                 // (fgmres_interface.h:136-138)
                 krylov7<double, 1>(C, x, b, C.w.p, C.scal.p + 16);
                 bytes += (3 * w8 + 4) * n;
-                KrylovScalars hs;
-                double tr2 = 0;
-                LSG_CUDA(cudaMemcpyAsync(&hs, ks, sizeof(hs), cudaMemcpyDeviceToHost, s));
-                LSG_CUDA(cudaMemcpyAsync(&tr2, C.scal.p + 16, sizeof(double), cudaMemcpyDeviceToHost, s));
+                LSG_CUDA(cudaMemcpyAsync(&C.host->st, &ks->st, sizeof(C.host->st), cudaMemcpyDeviceToHost, s));
+                LSG_CUDA(cudaMemcpyAsync(&C.host->r2, C.scal.p + 16, sizeof(double), cudaMemcpyDeviceToHost, s));
                 LSG_CUDA(cudaStreamSynchronize(s));
+                const KrylovScalars::State hs = C.host->st;
                 // FP64 reference semantics restart with the implicit norm |gamma|;
                 // with the FP32 preconditioner the restart is an iterative
                 // refinement step from the true FP64 residual, and the solve only
                 // ends when that true residual meets eps.
-                double g = refine ? std::sqrt(tr2) : std::fabs(hs.norm_r);
+                const double g = refine ? std::sqrt(C.host->r2) : std::fabs(hs.norm_r);
+                it = hs.it;
+                norm_r = g;
+                breakdown = hs.breakdown != 0;
                 if (finished) {
                     if (!(g > C.opt.eps) || !(hs.it < C.opt.max_it) || hs.breakdown) {
-                        hs.norm_r = g;
-                        LSG_CUDA(cudaMemcpyAsync(ks, &hs, sizeof(hs), cudaMemcpyHostToDevice, s));
+                        have_r2 = true;
                         break;
                     }
                     finished = false;
-                    hs.it++;
+                    it++;
                 }
-                hs.norm_r = g;
-                hs.invNormW = 1.0 / g;
-                hs.done = 0;
-                LSG_CUDA(cudaMemcpyAsync(ks, &hs, sizeof(hs), cudaMemcpyHostToDevice, s));
+                k_krylov_start<<<1, 32, 0, s>>>(ks, g, it, false);
+                LSG_CHECK_LAUNCH();
             }
         }
-        KrylovScalars hs;
-        LSG_CUDA(cudaMemcpyAsync(&hs, ks, sizeof(hs), cudaMemcpyDeviceToHost, s));
-        LSG_CUDA(cudaStreamSynchronize(s));
-        it = hs.it;
-        norm_r = hs.norm_r;
-        if (hs.breakdown) status = LSG_BREAKDOWN;
+    }
+    // the end of the solve's device time; the last scalars, the sweeps' error
+    // flag and (for the caller's statistics) the FP64 residual come back together
+    const bool iterated = it > 0;
+    LSG_CUDA(cudaEventRecord(C.ev1, s));
+    if (iterated && !have_r2)
+        LSG_CUDA(cudaMemcpyAsync(&C.host->st, &ks->st, sizeof(C.host->st), cudaMemcpyDeviceToHost, s));
+    ilu_fetch(C);
+    if (st && !have_r2) {
+        krylov7<double, 1>(C, x, b, C.t1.p, C.scal.p + 40);
+        LSG_CUDA(cudaMemcpyAsync(&C.host->r2, C.scal.p + 40, sizeof(double), cudaMemcpyDeviceToHost, s));
+    }
+    LSG_CUDA(cudaStreamSynchronize(s));
+    if (iterated) {
+        if (!have_r2) {
+            it = C.host->st.it;
+            norm_r = C.host->st.norm_r;
+            breakdown = C.host->st.breakdown != 0;
+        }
+        if (breakdown) status = LSG_BREAKDOWN;
         else if (!(norm_r <= C.opt.eps)) status = LSG_NOT_CONVERGED;
     }
-    ilu_check(C);
+    ilu_raise(C);
     if (st) {
         st->iterations = it;
         st->norm_r = norm_r;
         st->status = status;
+        st->true_residual = std::sqrt(C.host->r2);
     }
     C.bytes += bytes;
     return status;
@@ -1781,17 +1792,27 @@ static void ilu_tiles_apply(Context& C, const double* b, double* x, int withhold
     LSG_CHECK_LAUNCH();
 }
 
-// Raises the failure of a sweep in which a wait gave up.
+// The flag of a sweep in which a wait gave up, to the host; after the stream
+// is synchronised, its failure.
+static void ilu_fetch(Context& C)
+{
+    C.host->ilu_err = 0;
+    if (C.opt.precond != LSG_PC_ILU0 || !C.ilu_g.nc) return;
+    LSG_CUDA(cudaMemcpyAsync(&C.host->ilu_err, C.ilu_err.p, sizeof(int), cudaMemcpyDeviceToHost, C.s));
+}
+
+static void ilu_raise(Context& C)
+{
+    if (!C.host->ilu_err) return;
+    LSG_CUDA(cudaMemsetAsync(C.ilu_err.p, 0, sizeof(int), C.s));
+    throw Error{LSG_ERR_CUDA, "an ILU sweep's wait at a tile barrier gave up"};
+}
+
 static void ilu_check(Context& C)
 {
-    if (C.opt.precond != LSG_PC_ILU0 || !C.ilu_g.nc) return;
-    int e = 0;
-    LSG_CUDA(cudaMemcpyAsync(&e, C.ilu_err.p, sizeof(int), cudaMemcpyDeviceToHost, C.s));
+    ilu_fetch(C);
     LSG_CUDA(cudaStreamSynchronize(C.s));
-    if (e) {
-        LSG_CUDA(cudaMemsetAsync(C.ilu_err.p, 0, sizeof(int), C.s));
-        throw Error{LSG_ERR_CUDA, "an ILU sweep's wait at a tile barrier gave up"};
-    }
+    ilu_raise(C);
 }
 
 static void ilu_apply(Context& C, const double* b, double* x)
@@ -1916,10 +1937,14 @@ static int solve_device(Context& C, const double* b, double* x, lsg_stats* st)
     const long long l0 = g_launches;
     LSG_CUDA(cudaEventRecord(C.ev0, C.s));
     int rc;
-    if (C.opt.method == LSG_METHOD_BICGSTAB) rc = bicgstab(C, x, b, st);
-    else rc = fgmres(C, x, b, st);
-    LSG_CUDA(cudaEventRecord(C.ev1, C.s));
-    LSG_CUDA(cudaEventSynchronize(C.ev1));
+    const bool bicg = C.opt.method == LSG_METHOD_BICGSTAB;
+    if (bicg) {
+        rc = bicgstab(C, x, b, st);
+        LSG_CUDA(cudaEventRecord(C.ev1, C.s));
+        LSG_CUDA(cudaEventSynchronize(C.ev1));
+    } else {
+        rc = fgmres(C, x, b, st);           // records ev1, then synchronises
+    }
     float ms = 0;
     LSG_CUDA(cudaEventElapsedTime(&ms, C.ev0, C.ev1));
     if (st) {
@@ -1927,7 +1952,7 @@ static int solve_device(Context& C, const double* b, double* x, lsg_stats* st)
         st->bytes = C.bytes;
         st->vcycles = C.vcycles;
         st->kernel_launches = g_launches - l0;
-        st->true_residual = true_residual(C, x, b);
+        if (bicg) st->true_residual = true_residual(C, x, b);
     }
     return rc;
 }
@@ -1959,8 +1984,8 @@ static void context_init(Context& C, int device, cudaStream_t stream)
     C.scal.alloc(64);
     LSG_CUDA(cudaMemset(C.scal.p, 0, C.scal.bytes()));
     C.ks.alloc(1);
-    LSG_CUDA(cudaHostAlloc((void**)&C.hflag, 64, cudaHostAllocMapped));
-    C.hnorm = (double*)((char*)C.hflag + 8);
+    LSG_CUDA(cudaHostAlloc((void**)&C.host, sizeof(HostScalars), cudaHostAllocMapped));
+    std::memset(C.host, 0, sizeof(HostScalars));
     lsg_default_options(&C.opt);
 }
 
@@ -1973,8 +1998,8 @@ static cudaStream_t context_release(Context& C)
     }
     if (C.s) cudaStreamSynchronize(C.s);
     vcycle_graphs_release(C.mg);
-    if (C.hflag) cudaFreeHost(C.hflag);
-    C.hflag = nullptr;
+    if (C.host) cudaFreeHost(C.host);
+    C.host = nullptr;
     if (C.ev0) cudaEventDestroy(C.ev0);
     if (C.ev1) cudaEventDestroy(C.ev1);
     C.ev0 = C.ev1 = nullptr;
