@@ -1171,6 +1171,21 @@ static void prolong_level(const Dims& f, const Dims& c, bool even, const Transfe
     LSG_CHECK_LAUNCH();
 }
 
+// `sweeps` sweeps: one launch on 27-point levels whose iterate one CTA holds.
+template <typename T>
+static void gs_sweeps(const LevelT<T>& lv, const T* b, T* x, int sweeps, bool backward, cudaStream_t s)
+{
+    const Dims& d = lv.d;
+    const size_t sm = (size_t)(d.N + 2) * (d.M + 2) * (d.K + 2) * sizeof(T);
+    if (sweeps > 0 && lv.ol.n == 27 && lv.dict28.p && d.n() <= kGsSmallCells && sm <= kGsSmallSmem) {
+        launch_dep(k_gs_box27_small<T>, 1, 512, sm, s, d.N, d.M, d.K, sweeps, backward, lv.cls, lv.dict28.p,
+                   lv.gsdinv.p, b, x);
+        LSG_CHECK_LAUNCH();
+        return;
+    }
+    for (int it = 0; it < sweeps; it++) gs_sweep<T>(lv, b, x, backward, s);
+}
+
 // V(n_pre, n_post) cycle with the multi-colour Gauss-Seidel smoother (the
 // red-black variant): on the way down each level starts from zero, is
 // pre-smoothed, and restricts its residual; the coarsest level is solved by
@@ -1192,7 +1207,7 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
         const T* res = lv.r.p;
         if (npre > 0) {
             LSG_CUDA(cudaMemsetAsync(x, 0, f.n() * sizeof(T), s));
-            for (int it = 0; it < npre; it++) gs_sweep<T>(lv, lv.r.p, x, false, s);
+            gs_sweeps<T>(lv, lv.r.p, x, npre, false, s);
             // residual r - A x into c
             LSG_CUDA(cudaMemcpyAsync(lv.c.p, lv.r.p, f.n() * sizeof(T), cudaMemcpyDeviceToDevice, s));
             apply_resid<T>(lv, x, lv.c.p, s, 0);
@@ -1211,7 +1226,7 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
         T* x = (l == 0 && ch0) ? ch0 : lv.ch.p;
         if (npre > 0) prolong_level<T, true>(f, lev[l + 1].d, mg.agg[l], t, lev[l + 1].ch.p, x, nullptr, s);
         else prolong_level<T, false>(f, lev[l + 1].d, mg.agg[l], t, lev[l + 1].ch.p, x, lv.c.p, s);
-        for (int it = 0; it < npost; it++) gs_sweep<T>(lv, lv.r.p, x, true, s);
+        gs_sweeps<T>(lv, lv.r.p, x, npost, true, s);
     }
     C.vcycles++;
 }
