@@ -737,20 +737,34 @@ __global__ void k_restrict(int Nc, int Mc, int Kc, int N, int M, bool agglomerat
             acc += w * fine[f0 + NM + N];
             acc += w * fine[f0 + NM + N + 1];
         } else {
+            // the cell's three table rows first, then every gather: nothing
+            // waits for a table entry in between
+            int fx[4], fy[4], fz[4];
+            float wx[4], wy[4], wz[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                fx[q] = rx.f[4 * X + q];
+                fy[q] = ry.f[4 * Y + q];
+                fz[q] = rz.f[4 * Z + q];
+                wx[q] = rx.w[4 * X + q];
+                wy[q] = ry.w[4 * Y + q];
+                wz[q] = rz.w[4 * Z + q];
+            }
+#pragma unroll
             for (int a = 0; a < 4; a++) {
-                const int fz = rz.f[4 * Z + a];
-                if (fz < 0) continue;
-                const float wz = rz.w[4 * Z + a];
-                for (int b = 0; b < 4; b++) {
-                    const int fy = ry.f[4 * Y + b];
-                    if (fy < 0) continue;
-                    const float wy = ry.w[4 * Y + b];
+                T v[4][4];
+#pragma unroll
+                for (int b = 0; b < 4; b++)
+#pragma unroll
                     for (int q = 0; q < 4; q++) {
-                        const int fx = rx.f[4 * X + q];
-                        if (fx < 0) continue;
-                        acc += (T)(wz * wy * rx.w[4 * X + q]) * fine[(long long)fz * NM + fy * N + fx];
+                        const bool in = fz[a] >= 0 && fy[b] >= 0 && fx[q] >= 0;
+                        v[b][q] = in ? fine[(long long)fz[a] * NM + fy[b] * N + fx[q]] : (T)0;
                     }
-                }
+#pragma unroll
+                for (int b = 0; b < 4; b++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (fz[a] >= 0 && fy[b] >= 0 && fx[q] >= 0) acc += (T)(wz[a] * wy[b] * wx[q]) * v[b][q];
             }
         }
         coarse[I] = acc;
@@ -1521,12 +1535,43 @@ __global__ void __launch_bounds__(256) k_tdma_xwarp(int N, long long nlines, con
 // Coarsest-grid solve with the stored scaled/permuted LU factors
 // (LUDecompositionSparseMatrix DirectGauss/InverseGauss,
 // lu_decomposition_sparse_matrix.h:238-259): one thread, n is tiny.
+constexpr int kCoarseWarp = 48;           // coarsest systems up to this size are solved by a whole warp
+
 template <typename T>
 __global__ void k_coarse_solve(int n, const double* __restrict__ L, const double* __restrict__ U,
                                const double* __restrict__ scale, const int* __restrict__ perm,
                                const T* __restrict__ b, T* __restrict__ ch, double* __restrict__ work)
 {
     dep_begin(b, ch);
+    if (n <= kCoarseWarp) {
+        // lane i keeps the sums of rows i and i + 32 and takes the columns in
+        // turn: n dependent steps per triangle instead of n (n - 1) / 2
+        __shared__ double sL[kCoarseWarp * (kCoarseWarp + 1)], sU[kCoarseWarp * (kCoarseWarp + 1)];
+        constexpr int LD = kCoarseWarp + 1;
+        const int lane = threadIdx.x;
+        for (int e = lane; e < n * n; e += 32) {
+            const int i = e / n, j = e - i * n;
+            sL[j * LD + i] = L[e];
+            sU[j * LD + i] = U[e];
+        }
+        __syncwarp();
+        double x0 = lane < n ? scale[perm[lane]] * (double)b[perm[lane]] : 0.0;
+        double x1 = lane + 32 < n ? scale[perm[lane + 32]] * (double)b[perm[lane + 32]] : 0.0;
+        for (int j = 0; j < n; j++) {
+            const double y = __shfl_sync(0xffffffffu, j < 32 ? x0 : x1, j & 31);
+            if (lane > j && lane < n) x0 -= sL[j * LD + lane] * y;
+            if (lane + 32 > j && lane + 32 < n) x1 -= sL[j * LD + lane + 32] * y;
+        }
+        for (int j = n - 1; j >= 0; j--) {
+            if (lane == (j & 31)) (j < 32 ? x0 : x1) /= sU[j * LD + j];
+            const double z = __shfl_sync(0xffffffffu, j < 32 ? x0 : x1, j & 31);
+            if (lane < j) x0 -= sU[j * LD + lane] * z;
+            if (lane + 32 < j) x1 -= sU[j * LD + lane + 32] * z;
+        }
+        if (lane < n) ch[lane] = (T)(scale[lane] * x0);
+        if (lane + 32 < n) ch[lane + 32] = (T)(scale[lane + 32] * x1);
+        return;
+    }
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     double* y = work;
     double* z = work + n;
