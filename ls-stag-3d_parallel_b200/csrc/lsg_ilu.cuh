@@ -167,7 +167,7 @@ constexpr int kIluTY = 16, kIluTZ = 16, kIluT = kIluTY * kIluTZ;
 constexpr int kIluC = 4;                  // steps per chunk
 constexpr int kIluSlots = 3;              // chunks of factors and right-hand side in flight
 constexpr int kIluFaceSlots = 4;          // chunks of face values in flight
-constexpr int kIluThreads = kIluT + 64;   // line threads, the loading warp, the face warp
+constexpr int kIluThreads = kIluT + 96;   // line threads, the loading, face-in and face-out warps
 
 struct IluTiles {
     int N, M, K;
@@ -354,8 +354,9 @@ constexpr size_t ilu_sweep_smem()
 // waits for one that has not.  The loading warp brings chunks of coefficients
 // and right-hand sides (contiguous) into a ring in shared memory with bulk
 // copies; the face warp polls the two upstream tiles' face values of a chunk
-// and puts them into a ring of their own, one lane per face line; the line
-// threads take kIluC steps per chunk.  Each step also asks for the same
+// and puts them into a ring of their own, one lane per face line; the face-out
+// warp sends the tile's own face values on after each step; the line threads
+// take kIluC steps per chunk.  Each step also asks for the same
 // step's operands of the next chunk, in the shadow of its barrier, so a step
 // does not wait for them (0.52 against 0.56 ms for the momentum solve, 31.3
 // against 34.9 ms for BiCGStab).  Every wait ends after a second
@@ -471,16 +472,25 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
         return;
     }
 
+    if (warp == kIluT / 32 + 2) {                                 // the face-out warp
+        // after each step's barrier the tile's own two faces, for the tiles
+        // downstream: lanes 0..15 the y-face line tz = lane, lanes 16..31 the
+        // z-face line ty = lane - 16
+        const int q = lane & 15, e = FWD ? 15 : 0;
+        const double* src = sh + (lane < 16 ? e + kIluTY * q : q + kIluTY * e);
+        uint4* face = faces + ((long long)tile * S + (FWD ? 0 : S - 1)) * 32 + lane;
+        for (int st = 0; st < S; st++) {
+            asm volatile("bar.sync 1, %0;" ::"n"(kIluT + 32) : "memory");
+            ilu_face_store(face, src[((st + 1) & 1) * kIluT], tag);
+            face += FWD ? 32 : -32;
+        }
+        return;
+    }
+
     // the line threads
     const int ty = tid % kIluTY, tz = tid / kIluTY;
     const bool edge_y = FWD ? ty == 0 : ty == kIluTY - 1, edge_z = FWD ? tz == 0 : tz == kIluTZ - 1;
-    // this line is a face that the downstream tiles read
-    const bool out_y = FWD ? ty == kIluTY - 1 : ty == 0, out_z = FWD ? tz == kIluTZ - 1 : tz == 0;
-    // this step's places: the value, the two faces
-    const long long at0 = (long long)tile * S + (FWD ? 0 : S - 1);
-    double* vp = v + at0 * kIluT + tid;
-    uint4* fy = faces + at0 * 32 + tz;
-    uint4* fz = faces + at0 * 32 + 16 + ty;
+    double* vp = v + ((long long)tile * S + (FWD ? 0 : S - 1)) * kIluT + tid;   // this step's value
     constexpr int DIR = FWD ? 1 : -1;
     const double* ring_t = ring + tid;
     double a[kIluC][NK], r[kIluC], an[kIluC][NK], rn[kIluC];
@@ -531,12 +541,8 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
             // the next chunk's operands of this step, in the shadow of the barrier
             if (more) operands(slot, q, an[q], rn[q]);
             *vp = own;
-            if (out_y) ilu_face_store(fy, own, tag);
-            if (out_z) ilu_face_store(fz, own, tag);
             vp += DIR * kIluT;
-            fy += DIR * 32;
-            fz += DIR * 32;
-            asm volatile("bar.sync 1, %0;" ::"n"(kIluT) : "memory");
+            asm volatile("bar.sync 1, %0;" ::"n"(kIluT + 32) : "memory");
         }
         // this chunk's slots are free: its operands have been used, not only
         // asked for (an arrival may overtake shared loads in flight, and the
