@@ -10,6 +10,7 @@
 #include <cstring>
 #include <memory>
 #include <thread>
+#include <utility>
 
 #include "lsg_adlj_fused.cuh"
 #include "lsg_dict.cuh"
@@ -239,6 +240,7 @@ struct Context {
     DevBuf<uint4> ilu_faces;
     DevBuf<unsigned> ilu_ticket;
     unsigned ilu_sweeps_run = 0;
+    int ilu_withhold = -1;    // self-test: the ticket whose CTA leaves the next sweep at once
     double bytes = 0;
     int vcycles = 0;
     bool own_stream = true;
@@ -1799,13 +1801,13 @@ static void ilu_tile_sweep(Context& C, int withhold)
 }
 
 // x = U^{-1} L^{-1} b: b into the tiles' order, the two sweeps in place, back.
-static void ilu_tiles_apply(Context& C, const double* b, double* x, int withhold = -1)
+static void ilu_tiles_apply(Context& C, const double* b, double* x)
 {
     const IluTiles& g = C.ilu_g;
     const dim3 vg((unsigned)(g.nty * g.ntz), (unsigned)((g.steps() + 31) / 32), 4);
     k_ilu_tile_vector<true><<<vg, 256, 0, C.s>>>(g, b, C.ilu_v.p);
     LSG_CHECK_LAUNCH();
-    ilu_tile_sweep<true>(C, withhold);
+    ilu_tile_sweep<true>(C, std::exchange(C.ilu_withhold, -1));
     ilu_tile_sweep<false>(C, -1);
     k_ilu_tile_vector<false><<<vg, 256, 0, C.s>>>(g, C.ilu_v.p, x);
     LSG_CHECK_LAUNCH();
@@ -1906,6 +1908,16 @@ static int bicgstab(Context& C, double* x, const double* b, lsg_stats* st)
     }
     C.bytes += bytes;
     return status;
+}
+
+// x = P b on host vectors; raises the failure of an ILU sweep whose wait gave up.
+static void precond_apply_host(Context& C, const double* b, double* x)
+{
+    const long long n = C.n;
+    LSG_CUDA(cudaMemcpyAsync(C.bd.p, b, n * 8, cudaMemcpyHostToDevice, C.s));
+    precond_apply(C, C.bd.p, C.xd.p);
+    LSG_CUDA(cudaMemcpyAsync(x, C.xd.p, n * 8, cudaMemcpyDeviceToHost, C.s));
+    ilu_check(C);                             // synchronises
 }
 
 static void krylov_alloc(Context& C)
@@ -3377,11 +3389,7 @@ int lsg_precond_apply(lsg_ctx* h, const double* b, double* x)
     LSG_REQUIRE(C.have_setup, LSG_ERR_STATE, "lsg_setup must be called first");
     LSG_REQUIRE(b && x, LSG_ERR_ARG, "null vector");
     LSG_CUDA(cudaSetDevice(C.device));
-    const long long n = C.n;
-    LSG_CUDA(cudaMemcpyAsync(C.bd.p, b, n * 8, cudaMemcpyHostToDevice, C.s));
-    precond_apply(C, C.bd.p, C.xd.p);
-    LSG_CUDA(cudaMemcpyAsync(x, C.xd.p, n * 8, cudaMemcpyDeviceToHost, C.s));
-    LSG_CUDA(cudaStreamSynchronize(C.s));
+    precond_apply_host(C, b, x);
     return LSG_OK;
     LSG_API_END(h)
 }
@@ -3910,10 +3918,10 @@ int lsg_selftest_wait_limit(lsg_ctx* h)
     Context& C = h->c;
     LSG_REQUIRE(C.have_setup && C.opt.precond == LSG_PC_ILU0, LSG_ERR_STATE, "needs lsg_setup with ILU(0)");
     LSG_CUDA(cudaSetDevice(C.device));
-    LSG_CUDA(cudaMemsetAsync(C.t1.p, 0, C.n * sizeof(double), C.s));
     LSG_REQUIRE(C.ilu_g.nty * C.ilu_g.ntz >= 2, LSG_ERR_STATE, "the self-test needs a sweep of two tiles or more");
-    ilu_tiles_apply(C, C.t1.p, C.t2.p, 0);         // the first tile's CTA writes no face
-    ilu_check(C);                                  // throws: the others' wait ran out
+    std::vector<double> b((size_t)C.n, 0.0), x((size_t)C.n);
+    C.ilu_withhold = 0;                            // the first tile's CTA writes no face
+    precond_apply_host(C, b.data(), x.data());     // throws: the others' wait ran out
     return LSG_OK;
     LSG_API_END(h)
 }

@@ -146,11 +146,13 @@ def test_operator_outside_the_stencil_is_rejected():
 
 
 def test_bounded_wait_runs_out_and_is_reported():
-    """The one-launch ILU(0) sweep waits at a grid barrier between
-    hyperplanes for one second at most.  The self-test entry point runs it
-    with one CTA leaving before its first arrival: the others' wait runs
-    out, the kernel ends with its flag set, the call returns LSG_ERR_CUDA
-    with the reason, and the same context then solves normally."""
+    """The ILU(0) sweep's tiles wait for the face values of the tiles before
+    them for one second at most.  The self-test entry point runs one
+    application of the preconditioner, as lsg_precond_apply does, with the
+    first tile's CTA leaving at once: the others' waits run out, the kernel
+    ends with its flag set, the application itself returns LSG_ERR_CUDA with
+    the reason (a flag left set would fail the next, unrelated solve), and
+    the same context then applies and solves normally."""
     import time
 
     from lsstag_b200 import _lib as L
@@ -166,14 +168,17 @@ def test_bounded_wait_runs_out_and_is_reported():
     print(f"wait-limit self-test: rc {rc} after {dt:.2f} s: {msg}")
     assert rc == L.LSG_ERR_CUDA and "barrier" in msg
     assert 0.5 < dt < 60
-    # the context then solves as a fresh one does, to the bit
+    # the context then applies and solves as a fresh one does, to the bit
+    z = s.precondition(b)
     x = np.zeros(b.size)
     its = s.solve(b, x)
     s.close()
     f = S.ILUFGMRES()
     f.set_planes(P, dims, S.Task(eps=1e-8 * float(np.linalg.norm(b))))
+    zf = f.precondition(b)
     xf = np.zeros(b.size)
     itf = f.solve(b, xf)
     f.close()
+    assert np.array_equal(z, zf)
     assert its == itf and np.array_equal(x, xf) and np.all(np.isfinite(x))
 
