@@ -1727,13 +1727,25 @@ static void ilu_setup(Context& C)
         k_ilu_pivots<<<blocks, 256, 0, C.s>>>(lv, d.N, d.M, d.K, C.A7.p, C.iluU.p);
     }
     LSG_CHECK_LAUNCH();
-    // The tile layout pads x by 30 steps and y, z to whole tiles.  Grids that
-    // it would more than quadruple (a few cells in x, or slivers in y or z)
-    // and that hold enough for it to matter (8M positions, 0.7 GB) keep the
-    // natural order and one launch per hyperplane.
+    // The tile layout pads x by 30 steps and y, z to whole tiles.  Slabs pay
+    // for that in memory, not in time: four iterations on 1024 x 1024 x 3 (5.5
+    // positions a cell) take 5.2 ms, in natural order 124; 4 x 1024 x 600 (9
+    // a cell) 5.7 against 67.  So the tiles are used wherever the memory is
+    // there: layouts of up to two positions a cell (144 bytes) always, larger
+    // ones if they take at most half of what is free.  Otherwise the natural
+    // order, one launch per hyperplane.
     const IluTiles g = ilu_tiles(d.N, d.M, d.K);
     const long long pos = g.positions(), ntile = (long long)g.nty * g.ntz;
-    C.ilu_g = (pos <= 4 * n || pos <= (8LL << 20)) ? g : IluTiles{};
+    const size_t nface = (size_t)(ntile * g.steps() * 32);
+    bool tiles = pos <= 2 * n || C.ilu_faces.n == nface;   // or held already
+    if (!tiles) {
+        for (DevBuf<double>* q : {&C.ilu_facL, &C.ilu_facU, &C.ilu_v}) q->release();
+        C.ilu_faces.release();
+        size_t free = 0, total = 0;
+        LSG_CUDA(cudaMemGetInfo(&free, &total));
+        tiles = (size_t)pos * (kIluFwd + kIluBwd + 1) * sizeof(double) <= free / 2;
+    }
+    C.ilu_g = tiles ? g : IluTiles{};
     if (C.ilu_g.nc) {
         std::vector<int> order((size_t)ntile);
         size_t q = 0;
@@ -1744,7 +1756,7 @@ static void ilu_setup(Context& C)
         C.ilu_facL.alloc((size_t)pos * kIluFwd);
         C.ilu_facU.alloc((size_t)pos * kIluBwd);
         C.ilu_v.alloc((size_t)pos);
-        C.ilu_faces.alloc((size_t)(ntile * g.steps() * 32));
+        C.ilu_faces.alloc(nface);
         C.ilu_ticket.alloc(1);
         C.ilu_err.alloc(1);
         C.ilu_sweeps_run = 0;

@@ -1,6 +1,6 @@
 """ILU(0) applications at the edges of the sweeps' tiles (16 x 16 lines in y
-and z, chunks of 4 steps in x) and on a thin grid that keeps the natural-order
-sweeps, against the oracle's factorisation and triangular solves.
+and z, chunks of 4 steps in x), on slabs and in the natural order that tight
+memory leaves, against the oracle's factorisation and triangular solves.
 
 Bound: each entry of the two solves is a sum of at most three products and a
 quotient in FP64; on these diagonally dominant rows (off-diagonals at most
@@ -46,23 +46,46 @@ def test_ilu_apply_at_tile_edges(dims):
     s.close()
 
 
-def test_thin_grid_keeps_the_natural_order():
-    """A grid four cells wide in x that the tile layout would pad ninefold:
-    the same application, checked by its residual, L U x = b, on the operator
-    whose factors are known: L = I + strictly lower, U = D + strictly upper
-    of a decoupled-in-x operator (the fill-free case, L U = A)."""
+def _application(dims, P, b):
+    """One application, and the launches of a solve of two iterations."""
     from lsstag_b200 import solver as S
-    dims = (4, 1024, 600)
-    P = _planes(dims, 7)
-    P[2] = P[4] = P[0] = P[6] = 0.0          # only y couples: tridiagonal lines, ILU(0) is exact
     s = S.ILUFGMRES()
-    s.set_planes(P, dims)
-    b = np.random.default_rng(3).standard_normal(P.shape[1])
+    s.set_planes(P, dims, S.Task(eps=0.0, MAX_ITER=2))
     x = s.precondition(b)
-    r = b - s.apply(x)
+    s.solve(b, np.zeros(b.size))
+    launches = s.stats.kernel_launches
     s.close()
-    # a backward-stable tridiagonal solve: a few units of 1e-16 times |A||x|
-    assert np.abs(r).max() <= 1e-13 * np.abs(x).max()
+    return x, launches
+
+
+@pytest.mark.parametrize("dims,leave", [((4, 1024, 600), 2600 << 20), ((3, 64, 1400), 420 << 20)])
+def test_slabs_run_the_tiles_and_tight_memory_the_natural_order(dims, leave):
+    """Grids that the tile layout pads nine- and twelvefold run the tiled
+    sweeps (a solve of tens of launches, not of two per hyperplane and
+    application); with less than twice the layout's memory left on the GPU
+    they run in natural order: the same arithmetic, the same bits.  The
+    smaller one also against the oracle, every coupling present."""
+    import torch
+    P = _planes(dims, 7)
+    n = P.shape[1]
+    planes = sum(dims) - 2
+    b = np.random.default_rng(3).standard_normal(n)
+    x, launches = _application(dims, P, b)
+    assert launches < 100
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+    y, launches = _application(dims, P, b)
+    del hog
+    torch.cuda.empty_cache()
+    assert launches > 4 * planes             # two applications of two sweeps
+    assert np.array_equal(x, y)
+    if n < 500000:
+        import lsg_oracle as lo
+        from lsstag_b200 import cases
+        rp, col, val = cases.planes_to_csr(P, dims)
+        want = lo.ilu_solve(lo.ilu0(sp.csr_matrix((val, col, rp), shape=(n, n))), b)
+        assert np.abs(y - want).max() <= 1e-13 * np.abs(want).max()
 
 
 def test_concurrent_contexts_give_the_same_bits():
