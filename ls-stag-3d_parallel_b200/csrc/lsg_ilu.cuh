@@ -283,10 +283,13 @@ __device__ __forceinline__ void ilu_mbar_arrive(unsigned long long* bar)
 }
 
 // Waits for the phase of `bar` with this parity, for four seconds at most (the
-// face warp's polls, which these waits depend on, end after one): then the
-// error flag is set and the kernel runs on without waiting (wrong values,
-// reported by the solve), so no thread is left behind at a barrier.
-__device__ __forceinline__ void ilu_mbar_wait(unsigned long long* bar, unsigned parity, int* err, bool& gave_up)
+// face warps' polls, which these waits depend on, end after one), or, with
+// heed, until another wait of the launch has given up.  Then the error flag is
+// set and the kernel runs on without waiting (wrong values, reported by the
+// solve), so no thread is left behind at a barrier.  Waits for the kernel's own
+// copies do not heed the flag: a copy must not outlive its CTA.
+__device__ __forceinline__ void ilu_mbar_wait(unsigned long long* bar, unsigned parity, int* err, bool& gave_up,
+                                              bool heed = true)
 {
     unsigned long long t0 = 0;
     for (unsigned it = 0; !gave_up; it++) {
@@ -299,10 +302,10 @@ __device__ __forceinline__ void ilu_mbar_wait(unsigned long long* bar, unsigned 
             : "r"(ilu_smem(bar)), "r"(parity)
             : "memory");
         if (ok) break;
-        if ((it & 63) == 0) {
+        if ((it & 7) == 0) {
             const unsigned long long now = ilu_now();
             if (it == 0) t0 = now;
-            else if (now - t0 > 4000000000ull) {
+            else if (now - t0 > 4000000000ull || (heed && *(volatile int*)err != 0)) {
                 atomicExch(err, 1);
                 gave_up = true;
             }
@@ -359,8 +362,10 @@ constexpr size_t ilu_sweep_smem()
 // take kIluC steps per chunk.  Each step also asks for the same
 // step's operands of the next chunk, in the shadow of its barrier, so a step
 // does not wait for them (0.52 against 0.56 ms for the momentum solve, 31.3
-// against 34.9 ms for BiCGStab).  Every wait ends after a second
-// (ilu_mbar_wait); withhold >= 0 (the wait-limit self-test only): the CTA
+// against 34.9 ms for BiCGStab).  A poll for a face value gives up after a
+// second; then the other waits of the launch end too (ilu_mbar_wait), and CTAs
+// that start later leave at once, in this sweep and in those after it until
+// the flag is read; withhold >= 0 (the wait-limit self-test only): the CTA
 // with that ticket leaves at once and writes no face.
 //
 // The quotient by U_p comes from the rounded reciprocal r = 1 / U_p and one
@@ -386,9 +391,11 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
     unsigned long long* ffull = empty + kIluSlots;
     unsigned long long* fempty = ffull + kIluFaceSlots;
     __shared__ unsigned my;
+    __shared__ int dead;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         my = atomicAdd(ticket, 1u) - base;                        // base: the tickets of the earlier launches
+        dead = *(volatile int*)err;                               // a wait has given up: no more of them
         for (int k = 0; k < kIluSlots; k++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(full + k)), "r"(1) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(empty + k)), "r"(kIluT / 32)
@@ -403,7 +410,7 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
     }
     if (tid < kIluT) sh[tid] = sh[kIluT + tid] = 0.0;
     __syncthreads();
-    if ((int)my == withhold) return;
+    if (dead || (int)my == withhold) return;
     const int ntile = g.nty * g.ntz;
     const int tile = order[FWD ? (int)my : ntile - 1 - (int)my];
     const int ta = tile % g.nty, tb = tile / g.nty;
@@ -412,12 +419,18 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
 
     if (warp == kIluT / 32) {                                     // the loading warp
         if (lane != 0) return;
-        for (int c = 0; c < nc; c++) {
-            const int slot = c % kIluSlots, cf = FWD ? c : nc - 1 - c;
+        // A slot's barrier is armed again only when its copies have landed,
+        // whoever has given up: line threads that no longer wait free slots
+        // whose copies are still in flight, and a second arrival in that
+        // phase would break the barrier.
+        int issued = 0;
+        for (; issued < nc; issued++) {
+            const int c = issued, slot = c % kIluSlots, cf = FWD ? c : nc - 1 - c;
             if (c >= kIluSlots) {
+                bool late = false;
+                ilu_mbar_wait(full + slot, (unsigned)(c / kIluSlots - 1) & 1u, err, late, false);
                 ilu_mbar_wait(empty + slot, (unsigned)(c / kIluSlots - 1) & 1u, err, gave_up);
-                bool late = false;                                // a slot's copies end before the next ones start
-                if (gave_up) ilu_mbar_wait(full + slot, (unsigned)(c / kIluSlots - 1) & 1u, err, late);
+                if (late || gave_up) break;
             }
             double* dst = ring + (size_t)slot * (NK + 1) * CT;
             const long long chunk = (long long)tile * nc + cf;
@@ -427,9 +440,9 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
             ilu_bulk_load(dst, fac + chunk * NK * CT, NK * CT * sizeof(double), full + slot);
             ilu_bulk_load(dst + NK * CT, v + chunk * CT, CT * sizeof(double), full + slot);
         }
-        for (int c = max(0, nc - kIluSlots); c < nc; c++) {       // no copy outlives the CTA
+        for (int c = max(0, issued - kIluSlots); c < issued; c++) {   // no copy outlives the CTA
             bool late = false;
-            ilu_mbar_wait(full + c % kIluSlots, (unsigned)(c / kIluSlots) & 1u, err, late);
+            ilu_mbar_wait(full + c % kIluSlots, (unsigned)(c / kIluSlots) & 1u, err, late, false);
         }
         return;
     }

@@ -167,7 +167,9 @@ def test_bounded_wait_runs_out_and_is_reported():
     msg = s.ctx.lib.lsg_last_error(s.ctx.h).decode()
     print(f"wait-limit self-test: rc {rc} after {dt:.2f} s: {msg}")
     assert rc == L.LSG_ERR_CUDA and "barrier" in msg
-    assert 0.5 < dt < 60
+    # one second of polling; the waits that depend on it, and the CTAs and the
+    # backward sweep after it, end with it (8 s more where each waited itself)
+    assert 0.5 < dt < 4
     # the context then applies and solves as a fresh one does, to the bit
     z = s.precondition(b)
     x = np.zeros(b.size)
