@@ -1773,7 +1773,6 @@ static void ilu_setup(Context& C)
                                       (int)ilu_sweep_smem<false>()));
         LSG_CUDA(cudaStreamSynchronize(C.s));     // the order table goes out of scope
         C.iluL.release();
-        C.iluU.release();                         // the pivots are in facU
     } else {
         C.iluL.alloc(3 * n);
         k_ilu_lower<<<grid_for(n, 256), 256, 0, C.s>>>(d.N, d.M, d.K, C.A7.p, C.iluU.p, C.iluL.p);

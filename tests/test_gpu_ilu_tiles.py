@@ -88,6 +88,29 @@ def test_slabs_run_the_tiles_and_tight_memory_the_natural_order(dims, leave):
         assert np.abs(y - want).max() <= 1e-13 * np.abs(want).max()
 
 
+def test_rebuild_allocates_nothing():
+    """A rebuild on the same grid finds every array in place: it succeeds with
+    less than one vector's memory left."""
+    import torch
+    from lsstag_b200 import solver as S
+    dims = (96, 128, 128)
+    P = _planes(dims, 5)
+    s = S.ILUFGMRES()
+    s.set_planes(P, dims)
+    b = np.random.default_rng(4).standard_normal(P.shape[1])
+    x = s.precondition(b)
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free // (2 << 20) * (2 << 20) - (8 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        s.rebuildPreconditioner()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert np.array_equal(s.precondition(b), x)
+    s.close()
+
+
 def test_concurrent_contexts_give_the_same_bits():
     """Three contexts whose sweeps together have more tiles than the GPU has
     SMs, solving at once: every solve gives the bits of a solve alone (a ring
