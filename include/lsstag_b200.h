@@ -61,7 +61,7 @@ extern "C" {
 /* lsg_options.smoother */
 #define LSG_SMOOTHER_ADLJ 0   /* reference: damped z,y,x line Jacobi */
 #define LSG_SMOOTHER_RBGS 1   /* red-black point Gauss-Seidel (new variant) */
-#define LSG_ADLJ_AUTO 0       /* fused wherever a level's shape has the kernels, small FP64 grids aside */
+#define LSG_ADLJ_AUTO 0       /* as LSG_ADLJ_FUSED */
 #define LSG_ADLJ_REFERENCE 1  /* the reference's schedule: r -= A c, then the line solve */
 #define LSG_ADLJ_FUSED 2      /* ADLJ direction step as one kernel (residual formed in the line solve) */
 
@@ -92,9 +92,8 @@ typedef struct lsg_options {
                             (smoother_adlj_interface.h:66-77) everywhere.  The
                             two are equal in exact arithmetic (r = b - A ch
                             before every direction) and differ by rounding.
-                            LSG_ADLJ_AUTO (default): as LSG_ADLJ_FUSED, but the
-                            reference's schedule in the FP64 cycle of grids
-                            below 262144 cells. */
+                            LSG_ADLJ_AUTO (default): as LSG_ADLJ_FUSED, in both
+                            precisions and at every size. */
     int reserved[6];
 } lsg_options;
 

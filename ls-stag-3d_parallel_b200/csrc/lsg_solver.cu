@@ -1008,10 +1008,6 @@ static bool adlj_fused_level(const Dims& g, int noff, const std::vector<int>& of
 {
     if (o.smoother != LSG_SMOOTHER_ADLJ) return false;
     if (o.adlj_schedule == LSG_ADLJ_REFERENCE) return false;
-    // the default FP64 cycle of small grids keeps the reference's schedule: the
-    // rounding of the other one moved the drag gradient of a 64 x 32 x 32 flow,
-    // whose solves stop at an absolute 1e-9, by up to 1e-7 of its value
-    if (sizeof(T) == 8 && o.adlj_schedule == LSG_ADLJ_AUTO && g.n() < (1LL << 18)) return false;
     if (noff != 7 || off.size() < 3 || off[0] != 0 || off[1] != 0 || off[2] != -1) return false;
     if (g.N < 2 || g.M < 2 || g.K < 2 || !(xseg_cells(g.N) || xany_cells(g.N))) return false;
     return seg_cells<T>(g.M) != 0 && seg_cells<T>(g.K) != 0;

@@ -222,12 +222,18 @@ class GpuFlowOps:
     ILU(0)-FGMRES context per momentum equation and one per transposed
     momentum operator, and the loads context for the drag and its gradient.
 
+    The pressure cycle keeps the reference's smoother schedule: the solves
+    stop at an absolute tolerance, so the rounding of the cycle decides where,
+    and the fused schedule's moved a gradient by up to 1e-7 of its value
+    (64 x 32 x 32, solves to 1e-9).
+
     geom: FlowStepper's mesh arrays plus the loads inputs cells, dmax (delta_ib_max),
     dne (inv_delta_ib_ne), dtn (inv_delta_ib_tn) and, optionally, nodes and
     center (they enter the moments only, not the drag); par: FlowStepper's
     parameters plus fcoef and dt."""
 
     def __init__(self, geom: dict, dims, par: dict, device: int = 0):
+        from . import _lib as L
         from .loads import LoadsCalculator
         self.g, self.par = geom, par
         self.dims = tuple(int(v) for v in dims)
@@ -235,7 +241,7 @@ class GpuFlowOps:
         self.bc_lap = self.bc[[1, 8, 9, 16, 17]].copy()
         self.nu = float(par["nu"])
         ptask = S.Task(eps=par["eps"], MAX_ITER=int(par["max_it"]), FGMRES_RESTART_NUM=int(par["restart_p"]))
-        self.pres = S.MGFGMRES(device=device)
+        self.pres = S.MGFGMRES(device=device, adlj_schedule=L.ADLJ_REFERENCE)
         self.pres.set_geometry({k: geom[k] for k in ("celltype", "theta", "delta", "inv_mx", "inv_my", "inv_mz")},
                                self.dims, geom["pins"], task=ptask)
         self.pres.set_staggered_types(geom["xtype"], geom["ytype"], geom["ztype"])

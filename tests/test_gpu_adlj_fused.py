@@ -1,15 +1,14 @@
-"""The fused ADLJ direction step (LSG_ADLJ_FUSED, the default of the FP32
-cycle under LSG_ADLJ_AUTO: one kernel
-per direction forms the residual b - A ch inside its line solve and writes
+"""The fused ADLJ direction step (LSG_ADLJ_FUSED, and LSG_ADLJ_AUTO, the
+default, in both precisions: one kernel per direction forms the residual b - A ch inside its line solve and writes
 ch + omega T_d^{-1} (b - A ch)) against the reference's schedule
 (LSG_ADLJ_REFERENCE: r -= A c, c = omega T_d^{-1} r, ch += c as separate
 kernels, smoother_adlj_interface.h:66-77).  The two are equal in exact
 arithmetic, so one V-cycle agrees to rounding (a wrong coefficient, stride or
 buffer would show as an O(1) difference) and whole solves take the same
-iteration counts.  The fused kernels run on the levels with the 7-point
-stencil whose x-lines split into 8-cell segments over a power-of-two number
-of lanes (sphere16, the 128^3 four-sphere case); the coarse Galerkin levels
-keep the separate kernels."""
+iteration counts.  The fused kernels run on the level with the 7-point
+stencil (x-lines of up to 512 cells, by vectors where they split into 8-, 12-
+or 16-cell segments over a power-of-two number of lanes, by scalars
+otherwise); the coarse Galerkin levels keep the separate kernels."""
 import numpy as np
 import pytest
 
@@ -154,3 +153,36 @@ def test_fused_steps_profiled_128(case128):
     ms, by = ctypes.c_double(), ctypes.c_double()
     assert r.ctx.lib.lsg_profile_kernel(r.ctx.h, 9, 1, ctypes.byref(ms), ctypes.byref(by)) == L.LSG_ERR_STATE
     r.close()
+
+
+@pytest.mark.parametrize("dims", [(8, 6, 5), (32, 24, 20), (63, 30, 17), (64, 64, 64)])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_auto_fuses_at_every_size(prec, dims):
+    """LSG_ADLJ_AUTO runs the finest level's fused steps whatever the grid's
+    size: the same launches and bits as LSG_ADLJ_FUSED."""
+    from lsstag_b200 import _lib as L
+    from lsstag_b200 import solver as S
+    P, b = _long_case(dims)
+    out, launches = [], []
+    for sched in (L.ADLJ_AUTO, L.ADLJ_FUSED, L.ADLJ_REFERENCE):
+        s = S.MGFGMRES(mg_precision=L.FP32 if prec == "fp32" else L.FP64, adlj_schedule=sched)
+        s.set_planes(P, dims, S.Task(eps=0.0, MAX_ITER=2))
+        out.append(s.precondition(b))
+        s.solve(b, np.zeros(b.size))
+        launches.append(s.stats.kernel_launches)
+        s.close()
+    assert np.array_equal(out[0], out[1]) and launches[0] == launches[1] < launches[2]
+
+
+def test_gradient_operators_keep_the_reference_schedule():
+    """GpuFlowOps asks for it at every size (its solves stop at an absolute
+    tolerance, where the rounding of the cycle shows in the gradient)."""
+    from lsstag_b200 import _lib as L
+    from lsstag_b200 import cases
+    from lsstag_b200 import flow_adjoint as FA
+    dims, h = (32, 16, 16), 0.25
+    g, dims, par, _ = cases.flow_case_on_device(dims, (h, h, h), Re=100.0, dt=0.16 * h, eps=1e-9,
+                                                spheres=[(2.0, 2.0, 2.0, 0.5)])
+    ops = FA.GpuFlowOps(g, dims, dict(par, fcoef=float(g["fcoef"])))
+    assert ops.pres.options().adlj_schedule == L.ADLJ_REFERENCE
+    ops.close()
