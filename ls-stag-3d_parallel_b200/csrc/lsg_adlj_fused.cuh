@@ -75,7 +75,7 @@ __device__ __forceinline__ T resid7_at(int N, int M, int K, long long q, const i
 // the first right-hand side of the z-line
 // (x, y) is the residual at cell y*N*K + x, where the reference reads it
 // (smoother_adlj_z.h:54-58).  Shared memory: 4 W S values.
-template <typename T, int DIR, int SEG, int MAXT, int MINB, int VAR>
+template <typename T, int DIR, int SEG, int MAXT, int MINB, int VAR, bool DEP>
 __global__ void __launch_bounds__(MAXT, MINB)
     k_adlj_fused_seg(int N, int M, int K, bool zquirk, const int* __restrict__ cls, const T* __restrict__ dict,
                      const T* __restrict__ dinv, const T* __restrict__ b, const T* __restrict__ xin,
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         cl[u] = cls[i];
         dv[u] = dinv[i];
     }
-    dep_begin(b, xin, xout);                               // the operator does not wait for the step before
+    dep_begin<DEP>(b, xin, xout);                          // the operator does not wait for the step before
 #pragma unroll
     for (int u = 0; u < SEG; u++) {
         const int t = EXACT ? t0 + u : min(t0 + u, L - 1);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
 // for its end.  The eight scalar loads of a lane touch the same sectors as its
 // vectors would, through L1 (150 x 90 x 70 FP64 solve 6.93 ms against 7.30 with
 // the residual and the line solve as two launches on such lines).
-template <typename T, int SEG, bool ANY = false>
+template <typename T, int SEG, bool ANY, bool DEP>
 __global__ void __launch_bounds__(256) k_adlj_fused_xseg(int N, int M, int K, int P, const int* __restrict__ cls,
                                                           const T* __restrict__ dict, const T* __restrict__ dinv,
                                                           const T* __restrict__ b, const T* __restrict__ xin,
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) k_adlj_fused_xseg(int N, int M, int K, in
             cl[u] = cls[i];
             dv[u] = dinv[i];
         }
-        dep_begin(b, xin, xout);
+        dep_begin<DEP>(b, xin, xout);
 #pragma unroll
         for (int u = 0; u < SEG; u++) {
             const int i = min(base + u, last);
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) k_adlj_fused_xseg(int N, int M, int K, in
             cl[4 * k + 3] = c4.w;
         }
         load_seg<T, SEG>(dinv + base, dv);
-        dep_begin(b, xin, xout);
+        dep_begin<DEP>(b, xin, xout);
         load_seg<T, SEG>(b + base, bv);
         load_seg<T, SEG>(xin + base, xc);
         load_seg<T, SEG>(xin + base + bzm, zm);

@@ -229,20 +229,33 @@ struct HostScalars {
 // start.  Its kernels are launched with programmatic stream serialization:
 // the next one may be set up once every block of this one has started
 // (dep_begin's first half) and waits in dep_begin's second half until this
-// one's writes are visible.  Only grids that the GPU holds at once are launched
-// so: behind a grid of several waves there is nothing to hide, and the waiting
-// blocks take its slots (256^3 FP32 solve 26.7 against 26.3 ms; 64^3 2.86
-// against 2.94, 32 x 24 x 20 2.76 against 2.92, 150 x 90 x 70 6.89 against 7.36
-// ms with it).  Every kernel launched this way calls
-// dep_begin<pointers> before it reads or writes a vector; the pointers pass
-// through it so that no load of them is moved ahead of the wait.
+// one's writes are visible.  Grids of up to 2048 threads per SM only: behind
+// larger ones, several waves at these kernels' 64 to 255 registers, there is
+// nothing to hide, and the waiting blocks take slots (256^3 FP32 solve 26.7
+// against 26.3 ms; 64^3 2.86 against 2.94, 32 x 24 x 20 2.76 against 2.92,
+// 150 x 90 x 70 6.89 against 7.36 ms with it).  Every kernel launched this way
+// calls dep_begin<DEP>(pointers) before it reads or writes a vector; the
+// pointers pass through it so that no load of them is moved ahead of the wait.
+//
+// That also splits the kernel's loads into those before and those after, and
+// costs registers, launched dependently or not: the fused FP32 steps at 256^3
+// took 76, 111 and 131 us with it (x, y, z) and 72, 100 and 125 without, the
+// FP64 x and y steps 186 and 180 against 179 and 164.  The kernels that lose by
+// it have a second instance, DEP false, which larger grids get.
 // ---------------------------------------------------------------------------
-template <typename... P>
+template <bool DEP = true, typename... P>
 __device__ __forceinline__ void dep_begin(P&... ptr)
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    (([&] { asm volatile("" : "+l"(ptr)::"memory"); }()), ...);
+    if constexpr (DEP) {
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        (([&] { asm volatile("" : "+l"(ptr)::"memory"); }()), ...);
+    }
+}
+
+inline bool dep_grid(dim3 grid, dim3 block)
+{
+    return 1ull * grid.x * grid.y * grid.z * block.x * block.y * block.z <= 148ull * 2048;
 }
 
 template <typename... P, typename... A>
@@ -257,9 +270,18 @@ inline void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    const unsigned long long threads = 1ull * grid.x * grid.y * grid.z * block.x * block.y * block.z;
-    cfg.numAttrs = threads <= 148ull * 2048 ? 1 : 0;
+    cfg.numAttrs = dep_grid(grid, block) ? 1 : 0;
     LSG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
+// The instance with dep_begin on grids that are launched dependently, the one
+// without on larger ones.
+template <typename... P, typename... A>
+inline void launch_dep(void (*dep)(P...), void (*plain)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       A... args)
+{
+    if (dep_grid(grid, block)) launch_dep(dep, grid, block, smem, s, args...);
+    else plain<<<grid, block, smem, s>>>(static_cast<P>(args)...);
 }
 
 // ---------------------------------------------------------------------------

@@ -265,12 +265,12 @@ inline int zchunk_for(long long n) { return n >= (8LL << 20) ? 16 : (n >= (1LL <
 // (class index, r, the four lateral neighbours and the next plane) are all
 // issued before the arithmetic of those steps, so each thread has U cells of
 // loads in flight.  Terms are summed p, b, s, w, e, n, t.
-template <typename T, int MODE>
+template <typename T, int MODE, bool DEP>
 __global__ void __launch_bounds__(256) k_apply7z(int N, int M, int K, int zc, const int* __restrict__ cls,
                                                   const T* __restrict__ dict, const T* __restrict__ x,
                                                   T* __restrict__ r)
 {
-    dep_begin(x, r);
+    dep_begin<DEP>(x, r);
     constexpr int U = 4;
     const int ix = blockIdx.x * 32 + threadIdx.x;
     const int iy = blockIdx.y * 8 + threadIdx.y;
@@ -1199,7 +1199,7 @@ __device__ __forceinline__ void seg_scan(T& a, T& b, T* sA, T* sB)
 // S segment maps of a line are composed through shared memory by log-step
 // scans (SCAN), or by each thread walking the maps before its own.  Shared
 // memory: 4 W S values.
-template <typename T, int SEG, int MAXT, int MINB, bool SCAN = true>
+template <typename T, int SEG, int MAXT, int MINB, bool SCAN = true, bool DEP = true>
 __global__ void __launch_bounds__(MAXT, MINB) k_tdma_seg(LineGeom g, bool zquirk, const T* __restrict__ lo,
                                                          const T* __restrict__ dinv, const T* __restrict__ up,
                                                          const T* __restrict__ r, T* __restrict__ c,
@@ -1228,7 +1228,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_tdma_seg(LineGeom g, bool zquirk
         dv[u] = dinv[i];
         uv[u] = up[i];
     }
-    dep_begin(r, c, ch);                                   // the factors do not wait for the step before
+    dep_begin<DEP>(r, c, ch);                              // the factors do not wait for the step before
 #pragma unroll
     for (int u = 0; u < SEG; u++) {
         const int t = min(t0 + u, L - 1);

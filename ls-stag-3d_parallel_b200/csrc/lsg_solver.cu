@@ -871,10 +871,11 @@ static void apply_resid(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s, i
     const int zc = lv.ol.n == 27 ? (zc27 > 0 ? zc27 : (n >= (1LL << 20) ? 8 : zchunk_for(n))) : zchunk_for(n);
     const dim3 zb(32, 8), zg((lv.d.N + 31) / 32, (lv.d.M + 7) / 8, (lv.d.K + zc - 1) / zc);
     if (lv.ol.n == 7 && lv.off[0] == 0 && lv.off[2] == -1) {
-        if (mode == 0)
-            launch_dep(k_apply7z<T, 0>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
-        else
-            launch_dep(k_apply7z<T, 1>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
+        auto go = [&](auto dep, auto plain) {
+            launch_dep(dep, plain, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict, x, r);
+        };
+        if (mode == 0) go(k_apply7z<T, 0, true>, k_apply7z<T, 0, false>);
+        else go(k_apply7z<T, 1, true>, k_apply7z<T, 1, false>);
     } else if (lv.ol.n == 27 && lv.dict28.p) {
         if (mode == 0)
             launch_dep(k_apply27z<T, 0>, zg, zb, 0, s, lv.d.N, lv.d.M, lv.d.K, zc, lv.cls, lv.dict28.p, x, r);
@@ -906,19 +907,16 @@ static void line_solve(const LevelT<T>& lv, int d, bool zquirk, T omega, cudaStr
         };
         const bool aligned = ((reinterpret_cast<uintptr_t>(ch) | reinterpret_cast<uintptr_t>(lv.c.p)) & 15) == 0;
         const int P8 = xseg_p(8), P12 = xseg_p(12);
-        if (aligned && P8) {
-            const long long threads = nl * P8;
-            launch_dep(k_tdma_xseg<T, 8>, (unsigned)((threads + 255) / 256), 256, 0, s, 
-                g.N, P8, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p, ch, omega);
-        } else if (aligned && P12) {
-            const long long threads = nl * P12;
-            launch_dep(k_tdma_xseg<T, 12>, (unsigned)((threads + 255) / 256), 256, 0, s, 
-                g.N, P12, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p, ch, omega);
-        } else {
-            const int blocks = grid_for(nl * 32, 256, 148 * 64);
-            launch_dep(k_tdma_xwarp<T>, blocks, 256, 0, s, g.N, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p,
-                                                   ch, omega);
-        }
+        auto blocks = [&](int P) { return (unsigned)((nl * P + 255) / 256); };
+        auto go = [&](auto kernel, int P) {
+            launch_dep(kernel, blocks(P), 256, 0, s, g.N, P, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p, ch,
+                       omega);
+        };
+        if (aligned && P8) go(k_tdma_xseg<T, 8>, P8);
+        else if (aligned && P12) go(k_tdma_xseg<T, 12>, P12);
+        else
+            launch_dep(k_tdma_xwarp<T>, grid_for(nl * 32, 256, 148 * 64), 256, 0, s, g.N, nl, lv.lo[0].p, lv.dinv[0].p,
+                       lv.up[0].p, lv.r.p, lv.c.p, ch, omega);
     } else {
         LineGeom lg{g.N, g.M, g.K, d};
         constexpr int MAXT = sizeof(T) == 4 ? 512 : 256;
@@ -939,27 +937,24 @@ static void line_solve(const LevelT<T>& lv, int d, bool zquirk, T omega, cudaStr
         // CTAs per SM instead of one 126-register CTA of 8-cell segments:
         // 246 against 276 us at 256^3, measured); form 2 forces them
         const bool seg4 = (form == 2 || (form == 0 && sizeof(T) == 8 && d == 2)) && 8 * S4 <= 512;
+        auto go = [&](auto kernel, auto plain, int W, int S) {
+            const unsigned blocks = (unsigned)((long long)((g.N + W - 1) / W) * rows);
+            launch_dep(kernel, plain, blocks, dim3(W, S), 4 * (size_t)W * S * sizeof(T), s, lg, d == 2 && zquirk,
+                       lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
+        };
         if (seg4) {
-            const long long blocks = (long long)((g.N + 7) / 8) * rows;
-            launch_dep(k_tdma_seg<T, 4, 512, 2>, (unsigned)blocks, dim3(8, S4), 4 * (size_t)8 * S4 * sizeof(T), s, 
-                lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
+            // (with dep_begin's wait in it 257 us)
+            go(k_tdma_seg<T, 4, 512, 2>, k_tdma_seg<T, 4, 512, 2, true, false>, 8, S4);
         } else if (8 * S8 <= MAXT && (S8 <= 32 || 8 * S12 > MAXT)) {
-            const int W = pick_w(S8);
-            const long long blocks = (long long)((g.N + W - 1) / W) * rows;
-            if (walk)
-                launch_dep(k_tdma_seg<T, 8, MAXT, 2, false>, (unsigned)blocks, dim3(W, S8), 4 * (size_t)W * S8 * sizeof(T), s, 
-                    lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
-            else
-                launch_dep(k_tdma_seg<T, 8, MAXT, 2>, (unsigned)blocks, dim3(W, S8), 4 * (size_t)W * S8 * sizeof(T), s, 
-                    lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
+            // (no second instance: at 256^3 the split loads measured 147
+            // against 154 us, FP64 y, and 90 against 97, FP32 z)
+            if (walk) go(k_tdma_seg<T, 8, MAXT, 2, false>, k_tdma_seg<T, 8, MAXT, 2, false>, pick_w(S8), S8);
+            else go(k_tdma_seg<T, 8, MAXT, 2>, k_tdma_seg<T, 8, MAXT, 2>, pick_w(S8), S8);
         } else if (sizeof(T) == 4 && 8 * S12 <= MAXT) {
-            const int W = pick_w(S12);
-            const long long blocks = (long long)((g.N + W - 1) / W) * rows;
-            launch_dep(k_tdma_seg<T, 12, MAXT, 1>, (unsigned)blocks, dim3(W, S12), 4 * (size_t)W * S12 * sizeof(T), s, 
-                lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
+            go(k_tdma_seg<T, 12, MAXT, 1>, k_tdma_seg<T, 12, MAXT, 1>, pick_w(S12), S12);
         } else {
-            launch_dep(k_tdma_strided<T>, grid_for(lg.nlines(), 128, 148 * 64), 128, 0, s, 
-                lg, d == 2 && zquirk, lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
+            launch_dep(k_tdma_strided<T>, grid_for(lg.nlines(), 128, 148 * 64), 128, 0, s, lg, d == 2 && zquirk,
+                       lv.lo[d].p, lv.dinv[d].p, lv.up[d].p, lv.r.p, lv.c.p, ch, omega);
         }
     }
     LSG_CHECK_LAUNCH();
@@ -1032,14 +1027,17 @@ static void launch_fused_seg(const LevelT<T>& lv, bool zq, T omega, cudaStream_t
     const unsigned blocks = (unsigned)((long long)((g.N + W - 1) / W) * rows);
     const dim3 blk(W, S);
     const size_t sm = 4 * (size_t)W * S * sizeof(T);       // scan buffers
-    const T* dict = lv.dict;
+    // the large grids' instance; the FP64 z step is faster with its loads
+    // split (211 against 216 us at 256^3), the walked form (VAR 0) has one
+    constexpr bool PLAIN = VAR == 0 || (sizeof(T) == 8 && DIR == 2);
+    auto go = [&](auto dep, auto plain) {
+        launch_dep(dep, plain, blocks, blk, sm, s, g.N, g.M, g.K, zq, lv.cls, lv.dict, dinv, lv.r.p, xin, xout, omega);
+    };
     if (seg == 8) {
-        launch_dep(k_adlj_fused_seg<T, DIR, 8, MAXT, 2, VAR>, blocks, blk, sm, s, g.N, g.M, g.K, zq, lv.cls, dict, dinv,
-                                                                         lv.r.p, xin, xout, omega);
+        go(k_adlj_fused_seg<T, DIR, 8, MAXT, 2, VAR, true>, k_adlj_fused_seg<T, DIR, 8, MAXT, 2, VAR, PLAIN>);
     } else {
         if constexpr (sizeof(T) == 4)
-            launch_dep(k_adlj_fused_seg<T, DIR, 12, MAXT, 1, VAR>, blocks, blk, sm, s, g.N, g.M, g.K, zq, lv.cls, dict,
-                                                                              dinv, lv.r.p, xin, xout, omega);
+            go(k_adlj_fused_seg<T, DIR, 12, MAXT, 1, VAR, true>, k_adlj_fused_seg<T, DIR, 12, MAXT, 1, VAR, PLAIN>);
         else
             throw Error{LSG_ERR_STATE, "no fused line kernel for this line length"};
     }
@@ -1061,15 +1059,15 @@ static void adlj_fused_step(const LevelT<T>& lv, int d, bool zquirk, T omega, cu
         int P = 1;
         while (P * seg < g.N) P *= 2;
         const unsigned blocks = (unsigned)(((long long)g.M * g.K * P + 255) / 256);
-        auto go = [&](auto kernel) {
-            launch_dep(kernel, blocks, 256, 0, s, g.N, g.M, g.K, P, lv.cls, lv.dict, dinv, b, xin, xout, omega);
+        auto go = [&](auto dep, auto plain) {
+            launch_dep(dep, plain, blocks, 256, 0, s, g.N, g.M, g.K, P, lv.cls, lv.dict, dinv, b, xin, xout, omega);
         };
-        if (vec == 8) go(k_adlj_fused_xseg<T, 8>);
-        else if (vec == 12) go(k_adlj_fused_xseg<T, 12>);
-        else if (vec == 16) go(k_adlj_fused_xseg<T, 16>);
-        else if (seg == 8) go(k_adlj_fused_xseg<T, 8, true>);
-        else if (seg == 12) go(k_adlj_fused_xseg<T, 12, true>);
-        else go(k_adlj_fused_xseg<T, 16, true>);
+        if (vec == 8) go(k_adlj_fused_xseg<T, 8, false, true>, k_adlj_fused_xseg<T, 8, false, false>);
+        else if (vec == 12) go(k_adlj_fused_xseg<T, 12, false, true>, k_adlj_fused_xseg<T, 12, false, false>);
+        else if (vec == 16) go(k_adlj_fused_xseg<T, 16, false, true>, k_adlj_fused_xseg<T, 16, false, false>);
+        else if (seg == 8) go(k_adlj_fused_xseg<T, 8, true, true>, k_adlj_fused_xseg<T, 8, true, false>);
+        else if (seg == 12) go(k_adlj_fused_xseg<T, 12, true, true>, k_adlj_fused_xseg<T, 12, true, false>);
+        else go(k_adlj_fused_xseg<T, 16, true, true>, k_adlj_fused_xseg<T, 16, true, false>);
     } else {
         const bool zq = d == 2 && zquirk;
         if (scan) {

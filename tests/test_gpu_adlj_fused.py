@@ -131,6 +131,31 @@ def test_long_lines_fused_match_reference_schedule(dims, prec):
     assert abs(its[0] - its[1]) <= 1
 
 
+LARGE = [(256, 160, 130), (255, 150, 140), (384, 128, 112), (300, 150, 120), (512, 104, 100), (430, 112, 112)]
+
+
+@pytest.mark.parametrize("dims", LARGE)
+def test_large_grids_fused_match_reference_schedule(dims):
+    """Above 5 million cells, where the y and z steps test for one row per
+    warp and the kernels are launched without the dependent launches' wait:
+    x-lines of 8-, 12- and 16-cell segments, by vectors and by scalars, y-lines
+    of whole segments and not, z-lines of whole segments and not.  One V-cycle
+    against the reference's schedule, bounds as above."""
+    from lsstag_b200 import _lib as L
+    from lsstag_b200 import solver as S
+    P, b = _long_case(dims)
+    for prec, bound in ((L.FP64, 1e-12), (L.FP32, 1e-5)):
+        out = []
+        for sched in (L.ADLJ_FUSED, L.ADLJ_REFERENCE):
+            s = S.MGFGMRES(mg_precision=prec, adlj_schedule=sched)
+            s.set_planes(P, dims, S.Task(eps=1e-10 * float(np.linalg.norm(b))))
+            out.append(s.precondition(b))
+            s.close()
+        rel = np.linalg.norm(out[0] - out[1]) / np.linalg.norm(out[1])
+        print(f"{dims} {'fp64' if prec == L.FP64 else 'fp32'}: one V-cycle, fused vs reference schedule, {rel:.2e}")
+        assert rel <= bound
+
+
 def test_fused_steps_profiled_128(case128):
     """Kernel ids 9/10/11 (the fused x/y/z steps on the finest level) run
     and report their algorithmic bytes (4w + 4 per cell); the reference
