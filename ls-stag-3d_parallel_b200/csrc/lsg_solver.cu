@@ -1073,28 +1073,29 @@ static void adlj_fused_step(const LevelT<T>& lv, int d, bool zquirk, T omega, cu
         if (scan) {
             // y-lines that split into whole segments drop the line-end guards
             // (256^3 FP32: 112 against 131 us; the z step measured 140
-            // against 135 us that way and keeps them).  On grids of 4M cells
-            // and more FP32 y-lines and FP64 z-lines test for one row per
-            // warp (256^3: 102 against 111 and 214 against 225 us; FP32 z
-            // and FP64 y 145 against 125 and 191 against 164, and at 64^3
-            // FP32 y 6.0 against 4.5).
+            // against 135 us that way and keeps them).
+            // The test for one row per warp (VAR & 4), time with it and
+            // without.  FP64 z: never slower, 64^3 5.7 and 5.7 us, 128^3 25.4
+            // and 26.1, 150 x 90 x 70 14.7 and 14.7, 256^3 212 and 219.  FP32
+            // y with line-end guards, which it saves: 50 x 45 x 40 4.5 and
+            // 5.5, 150 x 90 x 70 9.6 and 10.8, 255 x 254 x 253 104 and 119.
+            // FP32 y of whole segments: it only saves loads, which cost little
+            // while the step's 20 bytes a cell stay in L2: 64^3 6.4 and 5.5,
+            // 128^3 13.1 and 12.3, 160^3 28.4 and 28.4, 256 x 160 x 128 36.5
+            // and 39.0, 192^3 53.3 and 58.6, 256^3 101 and 111; the line is
+            // drawn at 96 MB of the 126.  FP32 z and FP64 y: slower (256^3
+            // 145 against 125, 191 against 164).
             const int L = g.M;
             const int sgl = (sizeof(T) == 4 && 8 * ((L + 7) / 8) <= 512) ? 8 : seg_cells<T>(L);
-            const bool big = g.n() >= (1LL << 22);
-            if (d == 1) {
-                if constexpr (sizeof(T) == 4) {
-                    if (big && L % sgl == 0) launch_fused_seg<T, 1, 7>(lv, false, omega, s, dinv, xin, xout);
-                    else if (big) launch_fused_seg<T, 1, 5>(lv, false, omega, s, dinv, xin, xout);
-                }
-                if (sizeof(T) == 8 || !big) {
-                    if (L % sgl == 0) launch_fused_seg<T, 1, 3>(lv, false, omega, s, dinv, xin, xout);
-                    else launch_fused_seg<T, 1, 1>(lv, false, omega, s, dinv, xin, xout);
-                }
+            if constexpr (sizeof(T) == 4) {
+                if (d == 2) launch_fused_seg<T, 2, 1>(lv, zq, omega, s, dinv, xin, xout);
+                else if (L % sgl != 0) launch_fused_seg<T, 1, 5>(lv, false, omega, s, dinv, xin, xout);
+                else if (20 * g.n() < (96LL << 20)) launch_fused_seg<T, 1, 3>(lv, false, omega, s, dinv, xin, xout);
+                else launch_fused_seg<T, 1, 7>(lv, false, omega, s, dinv, xin, xout);
             } else {
-                if constexpr (sizeof(T) == 8) {
-                    if (big) launch_fused_seg<T, 2, 5>(lv, zq, omega, s, dinv, xin, xout);
-                }
-                if (sizeof(T) == 4 || !big) launch_fused_seg<T, 2, 1>(lv, zq, omega, s, dinv, xin, xout);
+                if (d == 2) launch_fused_seg<T, 2, 5>(lv, zq, omega, s, dinv, xin, xout);
+                else if (L % sgl != 0) launch_fused_seg<T, 1, 1>(lv, false, omega, s, dinv, xin, xout);
+                else launch_fused_seg<T, 1, 3>(lv, false, omega, s, dinv, xin, xout);
             }
         } else {
             if (d == 1) launch_fused_seg<T, 1, 0>(lv, false, omega, s, dinv, xin, xout);
