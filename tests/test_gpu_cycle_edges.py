@@ -53,21 +53,28 @@ def test_cycle_matches_oracle(dims):
         s.close()
 
 
+@pytest.mark.parametrize("schedule", ["fused", "reference"])
 @pytest.mark.parametrize("scale", [(1e3, 1.0, 1.0), (1.0, 1e3, 1.0), (1.0, 1.0, 1e3)])
-def test_strongly_coupled_lines(scale):
+@pytest.mark.parametrize("dims", [(64, 48, 40), (50, 45, 36)])
+def test_strongly_coupled_lines(dims, scale, schedule):
     """Lines coupled a thousand times more strongly along one direction: the
     segments' maps remember what enters them over the whole line, so the scans
-    run to their end."""
+    run to their end, in the fused steps and in the separate line solves."""
     import lsg_oracle as lo
+    from lsstag_b200 import _lib as L
     from lsstag_b200 import solver as S
-    P, A, b = _case((64, 48, 40), 3, scale)
-    want = lo.MultiGrid(A, (64, 48, 40)).apply(b)
-    s = S.MGFGMRES()
-    s.set_planes(P, (64, 48, 40))
-    got = s.precondition(b)
-    s.close()
-    # as above, times the lines' conditioning (about 1e3 / 1)
-    assert np.linalg.norm(got - want) <= 1e-10 * np.linalg.norm(want)
+    P, A, b = _case(dims, 3, scale)
+    want = lo.MultiGrid(A, dims).apply(b)
+    # as above, times the lines' conditioning (about 1e3 / 1); FP32: a
+    # rounding of 6e-8 times that a line solve, 6e-5, a few of which add up
+    for prec, bound in ((L.FP64, 1e-10), (L.FP32, 2e-4)):
+        s = S.MGFGMRES(mg_precision=prec, adlj_schedule=L.ADLJ_FUSED if schedule == "fused" else L.ADLJ_REFERENCE)
+        s.set_planes(P, dims)
+        got = s.precondition(b)
+        s.close()
+        rel = np.linalg.norm(got - want) / np.linalg.norm(want)
+        print(f"{dims} {scale} {schedule} {'fp64' if prec == L.FP64 else 'fp32'}: {rel:.1e}")
+        assert rel <= bound
 
 
 @pytest.mark.parametrize("dims", [(32, 32, 32), (24, 20, 12), (17, 19, 21), (64, 16, 8)])
