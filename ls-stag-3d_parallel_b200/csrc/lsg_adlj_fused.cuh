@@ -52,14 +52,6 @@ __device__ __forceinline__ T resid7_at_class(int N, int M, int K, long long q, i
     return b[q] - acc;
 }
 
-template <typename T, int RS>
-__device__ __forceinline__ T resid7_at(int N, int M, int K, long long q, const int* __restrict__ cls,
-                                       const T* __restrict__ dict, const T* __restrict__ b,
-                                       const T* __restrict__ x)
-{
-    return resid7_at_class<T, RS>(N, M, K, q, cls[q], dict, b, x);
-}
-
 // y-lines (DIR 1) and z-lines (DIR 2), segmented like k_tdma_seg: a CTA holds
 // W neighbouring lines (consecutive x) split into S = ceil(L/SEG) segments,
 // one thread per (line, segment).  Phase 1 loads the segment's row classes,

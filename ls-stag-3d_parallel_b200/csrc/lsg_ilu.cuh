@@ -154,9 +154,9 @@ __global__ void k_ilu_bwd(int level, int N, int M, int K, const double* __restri
 // at each tile border, until a grid has enough tiles to fill the memory pipe.
 // 16 x 16 lines keep the border crossings few (M/16 + K/16) with a barrier over
 // only eight warps.  Measured on a B200, a momentum solve of 127 x 64 x 64 (two
-// iterations): 0.52 ms against 2.30 ms with one cooperative launch and a grid
-// barrier per hyperplane; an ILU-BiCGStab solve of 64 x 48 x 40: 31 against
-// 139 ms.  The same bits.
+// iterations): 0.48 ms against 2.25 ms with one cooperative launch and a grid
+// barrier per hyperplane; an ILU-BiCGStab solve of 64 x 48 x 40: 29 against
+// 143 ms.  The same bits for finite values (see the quotient below).
 //
 // Storage follows the steps: position (tile, step, thread), so that every
 // stream is contiguous in the order in which it is used.  A tile has
@@ -372,7 +372,12 @@ constexpr size_t ilu_sweep_smem()
 // remainder step, q0 = a r, q = q0 + (a - q0 U_p) r, which rounds as the
 // division does (Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), in three
-// dependent operations instead of a division in the recurrence.
+// dependent operations instead of a division in the recurrence.  That holds
+// where a, q and the remainder are normal numbers.  A quotient that overflows
+// or an infinite a gives NaN instead of an infinity, a zero loses its sign, and
+// below 1e-290 or so the last bit may differ.  The padding multiplies by stored
+// zeros, so an infinity at a line's end also becomes NaN there, and in the
+// backward sweep of that line.  Either way the solve reports a breakdown.
 template <bool FWD>
 __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, const int* __restrict__ order,
                                                                  const double* __restrict__ fac, double* v,

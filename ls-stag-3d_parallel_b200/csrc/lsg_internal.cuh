@@ -211,12 +211,11 @@ struct KrylovScalars {
     int pad;
 };
 
-// The host's side of a solve in pinned memory: the flags that the kernels
+// The host's side of a solve in pinned memory: the flag that the kernels
 // write each step, and the targets of the copies at a solve's end.
 struct HostScalars {
     int flag;               // mapped: 2 finished, 1 not
     int ilu_err;
-    double norm;            // mapped: the step's residual estimate
     double r2;              // ||b - A x||^2
     KrylovScalars::State st;
 };

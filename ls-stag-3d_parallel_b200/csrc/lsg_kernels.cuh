@@ -1126,7 +1126,9 @@ __global__ void __launch_bounds__(128) k_tdma_strided(LineGeom g, bool zquirk, c
 
 // A segment map y = A + B y_in whose |B| is at most this forgets what enters
 // it: the term that a further scan step would add to A is below 2^-9 of the
-// rounding of the line's values (6e-8 and 1.1e-16 relative).
+// rounding (6e-8 and 1.1e-16 relative) of the line's largest values.  Values
+// smaller than those by as much lose it: a right-hand side of one cell leaves
+// exact zeros where the full scan leaves 1e-10 (1e-19) of the peak and less.
 template <typename T>
 __device__ __forceinline__ T scan_eps()
 {

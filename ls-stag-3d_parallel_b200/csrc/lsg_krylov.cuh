@@ -240,7 +240,6 @@ struct GivensArgs {
     int j, ldh, max_it;
     double eps;
     int* host_flag;        // mapped host memory
-    double* host_norm;
 };
 
 // Givens update of Hessenberg column j and the residual estimate
@@ -291,7 +290,6 @@ __device__ __forceinline__ void givens_update(const GivensArgs& g)
     }
     if (!(curA > 0.0) || isnan(gn)) ks->st.breakdown = 1;
     ks->done = done;
-    *(volatile double*)g.host_norm = gn;
     __threadfence_system();
     *(volatile int*)g.host_flag = done ? 2 : 1;
 }

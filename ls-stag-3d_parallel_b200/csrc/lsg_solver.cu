@@ -839,18 +839,17 @@ static void apply_box(const LevelT<T>& lv, const T* x, T* r, cudaStream_t s)
     const Dims& d = lv.d;
     const long long n = d.n();
     const int rx = -lv.off[0], ry = -lv.off[1], rz = -lv.off[2];   // the first offset is the box's corner
-    LSG_REQUIRE(rx >= 1 && rx <= 2 && ry >= 1 && ry <= 2 && rz >= 1 && rz <= 2 &&
+    LSG_REQUIRE(rx >= 1 && rx <= 2 && ry >= 1 && ry <= 2 && rz >= 1 && rz <= 2 && rx + ry + rz > 3 &&
                     lv.ol.n == (2 * rx + 1) * (2 * ry + 1) * (2 * rz + 1),
                 LSG_ERR_STATE, "unexpected coarse stencil");
     if (n < 32768) {
-        launch_dep(k_applybox8<T, MODE>, (unsigned)((n + 15) / 16), 128, 0, s, d.N, d.M, d.K, rx, ry, rz, lv.cls, lv.dict, x,
-                                                                      r);
+        launch_dep(k_applybox8<T, MODE>, (unsigned)((n + 15) / 16), 128, 0, s, d.N, d.M, d.K, rx, ry, rz, lv.cls,
+                   lv.dict, x, r);
         return;
     }
     const dim3 b(32, 4), g((d.N + 31) / 32, (d.M + 3) / 4, std::min(d.K, 65535));
     auto go = [&](auto kernel) { launch_dep(kernel, g, b, 0, s, d.N, d.M, d.K, lv.cls, lv.dict, x, r); };
-    switch (rx * 4 + ry * 2 + rz - 7) {
-    case 0: go(k_applybox<T, MODE, 1, 1, 1>); break;
+    switch (rx * 4 + ry * 2 + rz - 7) {                    // 1, 1, 1 has 27 points: k_apply27z
     case 1: go(k_applybox<T, MODE, 1, 1, 2>); break;
     case 2: go(k_applybox<T, MODE, 1, 2, 1>); break;
     case 3: go(k_applybox<T, MODE, 1, 2, 2>); break;
@@ -909,8 +908,8 @@ static void line_solve(const LevelT<T>& lv, int d, bool zquirk, T omega, cudaStr
         const int P8 = xseg_p(8), P12 = xseg_p(12);
         auto blocks = [&](int P) { return (unsigned)((nl * P + 255) / 256); };
         auto go = [&](auto kernel, int P) {
-            launch_dep(kernel, blocks(P), 256, 0, s, g.N, P, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p, ch,
-                       omega);
+            launch_dep(kernel, blocks(P), 256, 0, s, g.N, P, nl, lv.lo[0].p, lv.dinv[0].p, lv.up[0].p, lv.r.p, lv.c.p,
+                       ch, omega);
         };
         if (aligned && P8) go(k_tdma_xseg<T, 8>, P8);
         else if (aligned && P12) go(k_tdma_xseg<T, 12>, P12);
@@ -1116,14 +1115,14 @@ static void gs_sweep(const LevelT<T>& lv, const T* b, T* x, bool backward, cudaS
         const dim3 g((d.N / 2 + 1 + 31) / 32, (d.M + 7) / 8, d.K);
         for (int q = 0; q < 2; q++) {
             launch_dep(k_gs_rb7<T>, g, dim3(32, 8), 0, s, d.N, d.M, d.K, backward ? 1 - q : q, lv.cls, lv.dict,
-                                                  lv.gsdinv.p, b, x);
+                       lv.gsdinv.p, b, x);
             LSG_CHECK_LAUNCH();
         }
     } else if (lv.ol.n == 27 && lv.dict28.p) {
         const dim3 g(((d.N + 1) / 2 + 31) / 32, ((d.M + 1) / 2 + 7) / 8, (d.K + 1) / 2);
         for (int q = 0; q < 8; q++) {
             launch_dep(k_gs_box27<T>, g, dim3(32, 8), 0, s, d.N, d.M, d.K, backward ? 7 - q : q, lv.cls, lv.dict28.p,
-                                                    lv.gsdinv.p, b, x);
+                       lv.gsdinv.p, b, x);
             LSG_CHECK_LAUNCH();
         }
     } else {
@@ -1144,10 +1143,11 @@ static void restrict_level(const Dims& f, const Dims& c, bool even, const Transf
                            cudaStream_t s)
 {
     if (even && c.K <= 65535)
-        launch_dep(k_restrict_even<T>, dim3((c.N + 31) / 32, (c.M + 7) / 8, c.K), dim3(32, 8), 0, s, c.N, c.M, fine, coarse);
+        launch_dep(k_restrict_even<T>, dim3((c.N + 31) / 32, (c.M + 7) / 8, c.K), dim3(32, 8), 0, s, c.N, c.M, fine,
+                   coarse);
     else
-        launch_dep(k_restrict<T>, grid_for(c.n(), 256), 256, 0, s, c.N, c.M, c.K, f.N, f.M, even, t.R(0), t.R(1), t.R(2), fine,
-                                                          coarse);
+        launch_dep(k_restrict<T>, grid_for(c.n(), 256), 256, 0, s, c.N, c.M, c.K, f.N, f.M, even, t.R(0), t.R(1),
+                   t.R(2), fine, coarse);
     LSG_CHECK_LAUNCH();
 }
 
@@ -1166,8 +1166,8 @@ static void prolong_level(const Dims& f, const Dims& c, bool even, const Transfe
     } else {
         constexpr int PZ = 4;
         const dim3 g((f.N + 31) / 32, (f.M + 7) / 8, (f.K + PZ - 1) / PZ);
-        launch_dep(k_prolong<T, PZ, ADD>, g, dim3(32, 8), 0, s, f.N, f.M, f.K, c.N, c.M, t.P(0), t.P(1), t.P(2), coarse, ch,
-                                                        cc);
+        launch_dep(k_prolong<T, PZ, ADD>, g, dim3(32, 8), 0, s, f.N, f.M, f.K, c.N, c.M, t.P(0), t.P(1), t.P(2),
+                   coarse, ch, cc);
     }
     LSG_CHECK_LAUNCH();
 }
@@ -1217,8 +1217,8 @@ static void vcycle_rb(Context& C, std::vector<LevelT<T>>& lev, T* ch0)
         const TransferTabs& t = mg.tabs[l];
         restrict_level<T>(f, c, mg.agg[l], t, res, lev[l + 1].r.p, s);
     }
-    launch_dep(k_coarse_solve<T>, 1, 32, 0, s, mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
-                                       mg.dwork.p);
+    launch_dep(k_coarse_solve<T>, 1, 32, 0, s, mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p,
+               lev[L].ch.p, mg.dwork.p);
     LSG_CHECK_LAUNCH();
     for (int l = L - 1; l >= 0; l--) {
         LevelT<T>& lv = lev[l];
@@ -1264,11 +1264,13 @@ static void vcycle(Context& C, std::vector<LevelT<T>>& lev, T* ch0 = nullptr, bo
         restrict_level<T>(f, c, mg.agg[l], t, lev[l].r.p, lev[l + 1].r.p, s);
     }
     if (lt >= 0) {
-        if constexpr (sizeof(T) == 8) launch_dep(k_vcycle_tail<double>, 1, kTailThreads, mg.tail_smem64, s, mg.tail64.p);
-        else launch_dep(k_vcycle_tail<float>, 1, kTailThreads, mg.tail_smem32, s, mg.tail32.p);
+        if constexpr (sizeof(T) == 8)
+            launch_dep(k_vcycle_tail<double>, 1, kTailThreads, mg.tail_smem64, s, mg.tail64.p);
+        else
+            launch_dep(k_vcycle_tail<float>, 1, kTailThreads, mg.tail_smem32, s, mg.tail32.p);
     } else {
-        launch_dep(k_coarse_solve<T>, 1, 32, 0, s, mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p, lev[L].ch.p,
-                                           mg.dwork.p);
+        launch_dep(k_coarse_solve<T>, 1, 32, 0, s, mg.nc, mg.dL.p, mg.dU.p, mg.dscale.p, mg.dperm.p, lev[L].r.p,
+                   lev[L].ch.p, mg.dwork.p);
     }
     LSG_CHECK_LAUNCH();
     const T omega = (T)C.opt.omega;
@@ -1445,7 +1447,6 @@ static GivensArgs givens_args(const Context& C, int j)
     g.max_it = C.opt.max_it;
     g.eps = C.opt.eps;
     g.host_flag = &C.host->flag;
-    g.host_norm = &C.host->norm;
     return g;
 }
 
@@ -1565,7 +1566,8 @@ static int fgmres(Context& C, double* x, const double* b, lsg_stats* st)
                         const bool last = (i == j + 1);
                         k_mgs_step<<<gb, 256, 0, s>>>(n, Hj + (i - 1), C.V.p + (size_t)(i - 1) * C.ldv,
                                                      last ? C.w.p : C.V.p + (size_t)i * C.ldv, C.w.p, last, part, cnt,
-                                                     last ? &ks->normW2 : Hj + i, last ? givens_args(C, j) : GivensArgs{});
+                                                     last ? &ks->normW2 : Hj + i,
+                                                     last ? givens_args(C, j) : GivensArgs{});
                         LSG_CHECK_LAUNCH();
                         bytes += (last ? 3 : 4) * w8 * n;
                     }
