@@ -546,6 +546,12 @@ def main():
                          "launches": sum(r[2] for r in recs), "bytes": recs[-1][3], "true_res": recs[-1][4],
                          "norm_r": recs[-1][5], "x": x_dev.cpu().numpy(), "clocks": sampler.summary() if sampler else None,
                          "setup": {"operator_and_row_dictionary_ms": setup_ms[0], "hierarchy_ms": setup_ms[1]}}
+        # the finest level runs the fused direction steps (ids 9-11) unless
+        # its shape needs the separate residual and line-solve kernels
+        msk, byk = L.C.c_double(0), L.C.c_double(0)
+        fused = s.ctx.lib.lsg_profile_kernel(s.ctx.h, 9, 1, L.C.byref(msk), L.C.byref(byk)) == L.LSG_OK
+        results[name]["schedule"] = ("fused direction steps on the finest level (residual formed in the line solve)"
+                                     if fused else "reference schedule (r -= A c, then the line solve)")
         if name == "fp32":
             # dominant-kernel roofline (finest-level smoother/residual kernels)
             prof = {}
@@ -554,10 +560,6 @@ def main():
             names = {0: "adlj_xline_fp32", 1: "adlj_yline_fp32", 2: "adlj_zline_fp32", 3: "residual7_fp32",
                      5: "residual27_level1_fp32", 9: "adlj_fused_x_fp32", 10: "adlj_fused_y_fp32",
                      11: "adlj_fused_z_fp32"}
-            # the finest level runs the fused direction steps (ids 9-11) unless
-            # its shape needs the separate residual and line-solve kernels
-            msk, byk = L.C.c_double(0), L.C.c_double(0)
-            fused = s.ctx.lib.lsg_profile_kernel(s.ctx.h, 9, 1, L.C.byref(msk), L.C.byref(byk)) == L.LSG_OK
             for k in ((9, 10, 11, 5) if fused else (0, 1, 2, 3, 5)):
                 msk = L.C.c_double(0)
                 byk = L.C.c_double(0)
@@ -662,10 +664,7 @@ def main():
         "kernels": results["prof"],
         "setup_ms": {k: results[k]["setup"] for k in ("fp32", "fp64")},
         "rbgs_v22_fp32": rb,
-        "adlj_schedule": {"fp32": "fused direction steps on the finest level (residual formed in the line solve)"
-                          if any(k.startswith("adlj_fused") for k in results["prof"]) else
-                          "reference schedule (r -= A c, then the line solve)",
-                          "fp64": "as fp32"},
+        "adlj_schedule": {k: results[k]["schedule"] for k in ("fp32", "fp64")},
         "e2e": {"value": results["e2e_ms"] / world, "unit": "ms/solve", "h2d_bytes_per_step": 2 * 8 * n,
                 "d2h_bytes_per_step": 8 * n},
         "gpu_launches": results["fp32"]["launches"],
