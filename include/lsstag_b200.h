@@ -486,7 +486,7 @@ int lsg_apply(lsg_ctx* ctx, const double* x, double* y);
 /* x = M^{-1} b: one application of the configured preconditioner
    (MultiGridSolver::solve multigrid_solver.h:48-75 or the ILU(0) solves).
    Host buffers; for the FP32 multigrid the result is the FP32 cycle rounded
-   to FP64. */
+   to FP64.  LSG_ERR_CUDA if a wait of an ILU(0) sweep gave up. */
 int lsg_precond_apply(lsg_ctx* ctx, const double* b, double* x);
 
 /* Adjoint (no counterpart in the reference, which has no adjoint; built for
