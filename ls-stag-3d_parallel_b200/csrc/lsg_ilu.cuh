@@ -399,8 +399,9 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_tile_sweep(IluTiles g, cons
     __shared__ int dead;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
+        const int failed = *(volatile int*)err;                   // read first: both round trips at once
         my = atomicAdd(ticket, 1u) - base;                        // base: the tickets of the earlier launches
-        dead = *(volatile int*)err;                               // a wait has given up: no more of them
+        dead = failed;                                            // a wait has given up: no more of them
         for (int k = 0; k < kIluSlots; k++) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(full + k)), "r"(1) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ilu_smem(empty + k)), "r"(kIluT / 32)
