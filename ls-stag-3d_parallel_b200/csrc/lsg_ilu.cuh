@@ -236,8 +236,8 @@ __global__ void __launch_bounds__(256) k_ilu_tile_vector(IluTiles g, const doubl
                                                           double* __restrict__ dst)
 {
     __shared__ double sm[64][33];
-    const int S = g.nc * kIluC;
-    const int s0 = blockIdx.y * 32, zg = blockIdx.z, tile = blockIdx.x;
+    const int S = g.nc * kIluC, ns = (S + 31) / 32;
+    const int tile = blockIdx.x / ns, s0 = (blockIdx.x - tile * ns) * 32, zg = blockIdx.y;
     const int y0 = (tile % g.nty) * kIluTY, z0 = (tile / g.nty) * kIluTZ + zg * 4;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int l0 = threadIdx.x & 63, u0 = threadIdx.x >> 6;

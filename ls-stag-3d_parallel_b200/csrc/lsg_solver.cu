@@ -1812,7 +1812,7 @@ static void ilu_tile_sweep(Context& C, int withhold)
 static void ilu_tiles_apply(Context& C, const double* b, double* x)
 {
     const IluTiles& g = C.ilu_g;
-    const dim3 vg((unsigned)(g.nty * g.ntz), (unsigned)((g.steps() + 31) / 32), 4);
+    const dim3 vg((unsigned)(g.nty * g.ntz * ((g.steps() + 31) / 32)), 4);
     k_ilu_tile_vector<true><<<vg, 256, 0, C.s>>>(g, b, C.ilu_v.p);
     LSG_CHECK_LAUNCH();
     ilu_tile_sweep<true>(C, std::exchange(C.ilu_withhold, -1));
