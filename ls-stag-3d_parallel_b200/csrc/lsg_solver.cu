@@ -1026,8 +1026,8 @@ static void launch_fused_seg(const LevelT<T>& lv, bool zq, T omega, cudaStream_t
     const unsigned blocks = (unsigned)((long long)((g.N + W - 1) / W) * rows);
     const dim3 blk(W, S);
     const size_t sm = 4 * (size_t)W * S * sizeof(T);       // scan buffers
-    // the large grids' instance; the FP64 z step is faster with its loads
-    // split (211 against 216 us at 256^3), the walked form (VAR 0) has one
+    // the large grids' instance.  The FP64 z step keeps the split loads (256^3
+    // 212 against 219 us, 192^3 112 against 111), the walked form (VAR 0) too.
     constexpr bool PLAIN = VAR == 0 || (sizeof(T) == 8 && DIR == 2);
     auto go = [&](auto dep, auto plain) {
         launch_dep(dep, plain, blocks, blk, sm, s, g.N, g.M, g.K, zq, lv.cls, lv.dict, dinv, lv.r.p, xin, xout, omega);
